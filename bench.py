@@ -48,7 +48,7 @@ ALG = {"fp32": {"tdgl": 14 * 4 + 4, "pcg": 10 * 4 + 4, "ref": 28},
 # The per-kernel algorithmic bytes of the roofline line (by kernel):
 #   tdgl -> ALG tdgl; setup (first refinement pass; FP64: the RHS) and update
 #   (update pass) -> ALG ref (FP64 rhs: read Pm, write b: 3 s + 4 + s);
-#   spec (one direct solve) and pcg_iter / spmv+update -> ALG pcg;
+#   spec (one direct solve) and pcg_iter (one PCG iteration) -> ALG pcg;
 #   tdgl_check (the TDGL step that also forms the previous step's deferred
 #   check, one refinement pass's work) -> ALG tdgl + ALG ref.
 # Bytes the kernels as designed move per launch (what they read and write,
@@ -58,10 +58,9 @@ DESIGN_BYTES = {
     "fp32": {"tdgl": 6 * 4 * 2 + 8 + 4 + 2 * 8 + 8, "tdgl_check": 6 * 4 * 2 + 8 + 4 + 2 * 8 + 8 + 4 + 4 + 8,
              "setup": 8 + 12 + 4, "update": 8 + 4 + 4 + 4 + 8,
              "pcg_iter": 7 * 4 + 5 * 4, "spmv32": 4 * 4 + 2 * 4, "update32": 5 * 4 + 2 * 4, "spec": 40},
-    "fp64": {"tdgl": 6 * 8 * 2 + 8 + 4, "setup": 24 + 8 + 4 + 8 + 8, "spmv": 8 * 3 + 4 + 16,
-             "update": 5 * 8 + 2 * 8},
+    "fp64": {"tdgl": 6 * 8 * 2 + 8 + 4, "setup": 24 + 8 + 4 + 8 + 8, "pcg_iter": 6 * 8 + 5 * 8 + 8 + 4},
 }
-KERNELS = {"fp32": ["tdgl", "setup", "pcg_iter"], "fp64": ["tdgl", "setup", "spmv", "update"]}
+KERNELS = {"fp32": ["tdgl", "setup", "pcg_iter"], "fp64": ["tdgl", "setup", "pcg_iter"]}
 
 
 def alg_bytes(mode: str, kernel: str) -> int:
@@ -75,10 +74,6 @@ def alg_bytes(mode: str, kernel: str) -> int:
         return a["ref"]
     if mode == "fp64" and kernel == "setup":
         return 3 * 8 + 4 + 8
-    if mode == "fp64" and kernel == "spmv":
-        return 8 + 4 + 8                      # the SpMV part of one iteration
-    if mode == "fp64" and kernel == "update":
-        return a["pcg"] - (8 + 4 + 8)         # the update part
     return a["pcg"]                           # spec, pcg_iter, spmv32 + update32
 
 
@@ -451,7 +446,7 @@ def run_ours(args):
             "step_model": "B_tdgl + n_iter B_pcg + n_ref B_ref = %d + %.2f x %d + %.2f x %d" % (
                 ALG[mode]["tdgl"], n_iter, ALG[mode]["pcg"], n_ref, ALG[mode]["ref"])}
     if fp64:
-        launches = int(K * 3 + 2 * it.sum())
+        launches = int(K * 3)                 # TDGL, RHS, the persistent PCG
     elif deferred:
         # TDGL (with the previous step's check), the passes but that check,
         # five per direct solve; after the step loop the last check's pass and

@@ -365,7 +365,7 @@ extern "C" cmsl_status cmsl_film_loop_gradient(cmsl_film *f, int n_steps, const 
     }
     *loss = L / n_rows;
 
-    // ---- adjoint solve graph: k_adj_rhs -> WHILE { k_spmv -> k_update } on mu
+    // ---- adjoint solve graph: k_adj_rhs -> the PCG on mu
     cudaGraph_t g = nullptr;
     cudaGraphExec_t gx = nullptr;
     struct GraphGuard {
@@ -382,7 +382,7 @@ extern "C" cmsl_status cmsl_film_loop_gradient(cmsl_film *f, int n_steps, const 
     if (dep) {
         CK(cudaGraphCreate(&g, 0));
         cudaGraphConditionalHandle h = 0;
-        CK(cudaGraphConditionalHandleCreate(&h, g, 0, cudaGraphCondAssignDefault));
+        if (!e->pcg64) CK(cudaGraphConditionalHandleCreate(&h, g, 0, cudaGraphCondAssignDefault));
         Dev da = e->dev(1, h, 0);
         da.phi[0] = mu;
         da.solve = sadj;
@@ -392,9 +392,13 @@ extern "C" cmsl_status cmsl_film_loop_gradient(cmsl_film *f, int n_steps, const 
         cudaGraphNode_t n_rhs, n_loop, n_sp, n_up;
         cudaGraph_t body;
         TRY(add_kernel(g, &n_rhs, nullptr, 0, (void *)k_adj_rhs, nit, NT, a_rhs));
-        TRY(add_while(g, &n_loop, &n_rhs, 1, h, &body));
-        TRY(add_kernel(body, &n_sp, nullptr, 0, (void *)k_spmv<double, Fast>, nit, NT, a_pcg));
-        TRY(add_kernel(body, &n_up, &n_sp, 1, (void *)k_update<double, Fast, false>, nit, NT, a_pcg));
+        if (e->pcg64) {
+            TRY(add_pcg64(g, &n_loop, &n_rhs, e, da));
+        } else {
+            TRY(add_while(g, &n_loop, &n_rhs, 1, h, &body));
+            TRY(add_kernel(body, &n_sp, nullptr, 0, (void *)k_spmv<double, Fast>, nit, NT, a_pcg));
+            TRY(add_kernel(body, &n_up, &n_sp, 1, (void *)k_update<double, Fast, false>, nit, NT, a_pcg));
+        }
         CK(cudaGraphInstantiate(&gx, g, 0));
     }
     const Dev d0 = e->dev(0);

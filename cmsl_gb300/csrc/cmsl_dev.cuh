@@ -43,6 +43,7 @@ template <int TYc> struct TileShape {
     static constexpr int MINB = 1024 / NTt; // resident blocks per SM the kernels are built for
 };
 constexpr int TILE_YS[3] = {4, 8, 16};
+constexpr int P64_WORDS = 32;       // FP64 PCG: all-reduce words of a film (two sets, 128 bytes apart)
 constexpr int NPART = 8;            // doubles of partial sums per item
 
 constexpr uint32_t GID_MASK = 0x00ffffffu;
@@ -69,6 +70,8 @@ struct FilmDev {
     int sitem_begin, sitem_end; // the film's range of the FP32 stencil passes' items (Dev::sitems)
     int pb_begin, pb_end;       // persistent PCG: the film's block range of the cooperative grid
     int brick_begin, brick_end; // persistent PCG: the film's stencil bricks
+    int p64_rows, p64_nc;       // FP64 PCG: rows of a warp's units, and their z chunks (streaming form) or
+                                // planes (resident form)
     int dep_flag;
     int warm;                   // FP32_REFINED warm start: 0 previous phi, 1 linear, 2 quadratic, 3 cubic extrapolation
     int ref_id;                 // Neumann pinned cell (film-local)
@@ -196,7 +199,10 @@ struct Dev {
     int force;                  // run the PCG kernels whatever the flags (kernel timing)
     int step_end;               // a residual pass that leaves no film active also ends the step
     int defer;                  // films with defer_ok end a step on its direct solve (SolveDev::pending)
-    unsigned int *arrive;       // grid-barrier counter of the persistent PCG (or null)
+    union {
+        unsigned int *arrive;       // FP32: grid-barrier counter of the persistent PCG (or null)
+        unsigned long long *words;  // FP64: all-reduce words of the persistent PCG (or null), P64_WORDS per film
+    };
     cudaGraphConditionalHandle h_inner, h_outer;
     cudaGraphConditionalHandle h_steps;   // the graph's step loop (0: one step per launch)
     const FilmMaps *maps;       // [n_films] tensor maps (TMA stencil passes), or null

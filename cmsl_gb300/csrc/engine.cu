@@ -6,7 +6,7 @@
 // per-film quantity (solver scalars, convergence flags, waveform, sweep rows)
 // lives in per-film device slots.  A run is one CUDA graph launch: a WHILE
 // node over the steps whose body is one time step,
-//   CMSL_FP64:          k_tdgl -> k_rhs -> WHILE(inner){ k_spmv -> k_update } -> k_step_end
+//   CMSL_FP64:          k_tdgl -> k_rhs -> k_pcg64 (every iteration of every film; ends the step)
 //   CMSL_FP32_REFINED:  k_tdgl32 -> k_refine32 -> solve -> k_refine32
 //                       -> WHILE(outer){ solve -> k_refine32 }
 // where the FP32 inner solve is the direct spectral solve (films of one eps,
@@ -435,6 +435,20 @@ cmsl_status add_if(cudaGraph_t g, cudaGraphNode_t *node, const cudaGraphNode_t *
     return CMSL_OK;
 }
 
+// The FP64 PCG of every active film (d.step_end: it also ends the step).
+cmsl_status add_pcg64(cudaGraph_t g, cudaGraphNode_t *node, const cudaGraphNode_t *dep, const Engine *e, Dev d)
+{
+    Fields<double> F = e->fields<double>();
+    Pcg64 B = e->p64;
+    void *args[] = {&d, &F, &B};
+    TRY(add_kernel(g, node, dep, dep ? 1 : 0, e->p64_resident ? (void *)k_pcg64r : (void *)k_pcg64, e->p64_grid, P64_NT,
+                   args, 0));
+    cudaLaunchAttributeValue av{};
+    av.cooperative = 1;
+    CK(cudaGraphKernelNodeSetAttribute(*node, cudaLaunchAttributeCooperative, &av));
+    return CMSL_OK;
+}
+
 // Arguments must outlive graph instantiation only (node params are copied).
 cmsl_status build_graph(Engine *e)
 {
@@ -463,7 +477,7 @@ cmsl_status build_graph(Engine *e)
     const bool fp64 = e->precision == CMSL_FP64;
     cudaGraphNode_t n_tdgl, n_solve, n_end;
     if (!fp64 && e->any_dep) CK(cudaGraphConditionalHandleCreate(&h_outer, g, 1, cudaGraphCondAssignDefault));
-    if (fp64 && e->any_dep) CK(cudaGraphConditionalHandleCreate(&h_inner, g, 0, cudaGraphCondAssignDefault));
+    if (fp64 && e->any_dep && !e->pcg64) CK(cudaGraphConditionalHandleCreate(&h_inner, g, 0, cudaGraphCondAssignDefault));
     a.d = dev(h_inner, h_outer);
     void *args64[] = {&a.d, &a.F64};
     void *args32[] = {&a.d, &a.F32};
@@ -513,10 +527,17 @@ cmsl_status build_graph(Engine *e)
             cudaGraphNode_t n_rhs, n_sp, n_up;
             cudaGraph_t body;
             TRY(add_kernel(g, &n_rhs, &last, 1, (void *)k_rhs<double, Exact>, nit, NT, args64));
-            TRY(add_while(g, &n_solve, &n_rhs, 1, h_inner, &body));
-            TRY(add_kernel(body, &n_sp, nullptr, 0, (void *)k_spmv<double, Exact>, nit, NT, args64));
-            TRY(add_kernel(body, &n_up, &n_sp, 1, (void *)k_update<double, Exact, false>, nit, NT, args64));
-            last = n_solve;
+            if (e->pcg64) {
+                Dev dp = a.d;
+                dp.step_end = 1;
+                TRY(add_pcg64(g, &n_solve, &n_rhs, e, dp));
+                last = nullptr;
+            } else {
+                TRY(add_while(g, &n_solve, &n_rhs, 1, h_inner, &body));
+                TRY(add_kernel(body, &n_sp, nullptr, 0, (void *)k_spmv<double, Exact>, nit, NT, args64));
+                TRY(add_kernel(body, &n_up, &n_sp, 1, (void *)k_update<double, Exact, false>, nit, NT, args64));
+                last = n_solve;
+            }
         } else if (e->spectral || e->persistent) {
             // A step almost always takes two refinement passes (the warm
             // start's residual, then the check after one inner solve), so
@@ -799,6 +820,18 @@ cmsl_status launch_tdgl32(Engine *e, cudaStream_t st, const Dev &d, const Fields
     return CMSL_OK;
 }
 
+// The FP64 PCG of every active film, launched from the host.
+cmsl_status launch_pcg64(Engine *e, cudaStream_t st, const Dev &d, const Fields<double> &F64)
+{
+    Dev dd = d;
+    Fields<double> ff = F64;
+    Pcg64 B = e->p64;
+    void *args[] = {&dd, &ff, &B};
+    CK(cudaLaunchCooperativeKernel(e->p64_resident ? (void *)k_pcg64r : (void *)k_pcg64, dim3((unsigned)e->p64_grid),
+                                   dim3(P64_NT), args, 0, st));
+    return CMSL_OK;
+}
+
 // The direct spectral solve of the correction, launched from the host.
 cmsl_status spec_launch(Engine *e, cudaStream_t st, const Dev &d, const Fields<float> &F32)
 {
@@ -837,6 +870,7 @@ cmsl_status solve_direct(Engine *e, cudaStream_t st, const Dev &d, const Fields<
     if (e->precision == CMSL_FP64) {
         k_rhs<double, Exact><<<nit, NT, 0, st>>>(d, F64);
         CK(cudaGetLastError());
+        if (e->pcg64) return launch_pcg64(e, st, d, F64);
         for (int guard = 0;; ++guard) {
             TRY(read_flags(e, st, &act, nullptr));
             if (!act) break;
@@ -1112,6 +1146,79 @@ cmsl_status make_maps(Engine *e)
     return CMSL_OK;
 }
 
+// FP64 instructions of one iteration of a unit of R rows x zc planes: the
+// direction (own cells, y and x halos, the planes below and above), the rows,
+// the update.
+double pcg64_unit_cost(int R, int zc) { return R * (zc + 2) + 3.0 * zc + 13.0 * R * zc; }
+
+// The film's unit shape for the resident FP64 PCG on nb blocks, the smallest
+// that gives every unit a warp (more warps hide more latency: 96x80x20 takes
+// 9.0 us an iteration with 2 x 2, 13.7 with 2 x 4); false where none does.
+bool pcg64_plan_resident(FilmDev &fd, const FilmHost &h, int nb)
+{
+    static const int shapes[][2] = {{1, 1}, {1, 2}, {2, 2}, {2, 4}};
+    for (const auto &s : shapes) {
+        const long long units = (long long)((h.nx + 31) / 32) * ((h.ny + s[0] - 1) / s[0]) * ((h.nz + s[1] - 1) / s[1]);
+        if (units > (long long)nb * P64_NW) continue;
+        fd.p64_rows = s[0];
+        fd.p64_nc = s[1];
+        return true;
+    }
+    return false;
+}
+
+// Units of the streaming form's phase S on nb blocks: rows a warp owns and z
+// chunks; about 800 + 150 cycles a plane of latency per round of units.
+void pcg64_plan(FilmDev &fd, const FilmHost &h, int nb)
+{
+    double best = 0.0;
+    for (int R = 1; R <= 4; R *= 2)
+        for (int nc = 1; nc <= h.nz; ++nc) {
+            const int zc = (h.nz + nc - 1) / nc;
+            const double units = (double)((h.nx + 31) / 32) * ((h.ny + R - 1) / R) * nc;
+            const double cost = std::ceil(units / nb) * pcg64_unit_cost(R, zc) * 16.0 +
+                                std::ceil(units / (nb * P64_NW)) * (800.0 + 150.0 * zc);
+            if (best == 0.0 || cost < best) {
+                best = cost;
+                fd.p64_rows = R;
+                fd.p64_nc = nc;
+            }
+        }
+}
+
+// Blocks of each depolarised film of a launch of `total` blocks: in
+// proportion to its cells, at most cap(film).
+template <class Cap> std::vector<int> share_blocks(const Engine *e, int total, Cap cap)
+{
+    const int n = e->n_films;
+    long long tot = 0;
+    for (const FilmHost &h : e->fh) tot += h.dep ? h.N : 0;
+    std::vector<int> nb((size_t)n, 0);
+    int sum = 0;
+    for (int fi = 0; fi < n; ++fi)
+        if (e->fh[fi].dep) {
+            nb[fi] = std::min(cap(fi), std::max(1, (int)((double)total * e->fh[fi].N / tot)));
+            sum += nb[fi];
+        }
+    while (sum > total) {                // films rounded up to one block: the largest give theirs
+        --*std::max_element(nb.begin(), nb.end());
+        --sum;
+    }
+    while (sum < total) {                // the rest to the most loaded films
+        int best = -1;
+        double load = 0.0;
+        for (int fi = 0; fi < n; ++fi) {
+            if (!nb[fi] || nb[fi] >= cap(fi)) continue;
+            const double l = (double)e->fh[fi].N / nb[fi];
+            if (l > load) { load = l; best = fi; }
+        }
+        if (best < 0) break;
+        ++nb[best];
+        ++sum;
+    }
+    return nb;
+}
+
 cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
 {
     for (int i = 0; i < n; ++i) TRY(check_desc(descs + i, i, n));
@@ -1194,6 +1301,22 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
         if (n > cg_per * cg_nsm) e->persistent = false;
     }
 
+    // FP64 PCG: one cooperative launch for every film, resident where every
+    // film's vectors fit the registers of its share of one block per SM
+    int p64_nsm = 0, p64_per = 0;
+    e->pcg64 = e->precision == CMSL_FP64 && e->any_dep && n <= CG_MAX_FILMS && !(tk && atoi(tk) != 0);
+    if (e->pcg64) {
+        int dev = 0, per1 = 0;
+        CK(cudaGetDevice(&dev));
+        CK(cudaDeviceGetAttribute(&p64_nsm, cudaDevAttrMultiProcessorCount, dev));
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&p64_per, k_pcg64, P64_NT, 0));
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per1, k_pcg64r, P64_NT, 0));
+        if (p64_per < 1 || per1 < 1) return fail(CMSL_ERR_CUDA, "FP64 PCG kernel cannot be resident");
+        p64_per = std::min(p64_per, P64_BPS);
+        p64_nsm = std::min(p64_nsm, P64_MAX_BLOCKS / P64_BPS);
+        if (n > p64_nsm) e->pcg64 = false;
+    }
+
     // grain ids are checked on the host (before any device work); the
     // per-cell codes, interface flags and material voxel counts are built on
     // the device below (build_film_codes); work items, film tables
@@ -1235,6 +1358,27 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
     // (one film: as many blocks as give every block the same brick count)
     std::vector<int4> bricks;
     std::vector<int> blk_film;
+    if (e->pcg64) {
+        // a contiguous block range per depolarised film, a warp's work of 32 cells a block at least
+        auto cap = [&](int fi) {
+            const FilmHost &h = e->fh[fi];
+            const long long rows = (long long)((h.nx + 31) / 32) * h.ny * h.nz;
+            return (int)std::min<long long>(P64_MAX_BLOCKS, (rows + P64_NW - 1) / P64_NW);
+        };
+        std::vector<int> nb = share_blocks(e, p64_nsm, cap);
+        const char *fs = getenv("CMSL_P64_STREAM");          // 1: the streaming form whatever the size
+        e->p64_resident = !(fs && atoi(fs) != 0);
+        for (int fi = 0; fi < n; ++fi)
+            if (nb[fi]) e->p64_resident = pcg64_plan_resident(fds[fi], e->fh[fi], nb[fi]) && e->p64_resident;
+        if (!e->p64_resident) nb = share_blocks(e, p64_nsm * p64_per, cap);
+        for (int fi = 0; fi < n; ++fi) {
+            fds[fi].pb_begin = (int)blk_film.size();
+            blk_film.insert(blk_film.end(), (size_t)nb[fi], fi);
+            fds[fi].pb_end = (int)blk_film.size();
+            if (nb[fi] && !e->p64_resident) pcg64_plan(fds[fi], e->fh[fi], nb[fi]);
+        }
+        e->p64_grid = (int)blk_film.size();
+    }
     if (e->persistent) {
         for (int fi = 0; fi < n; ++fi) {
             const FilmHost &h = e->fh[fi];
@@ -1339,6 +1483,21 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
     TRY(e->alloc(&e->d_p[0], e->esz * cells));
     TRY(e->alloc(&e->d_p[1], e->esz * cells));
     if (e->precision != CMSL_FP64) TRY(e->alloc(&e->d_x, e->esz * cells));
+    if (e->pcg64) {
+        Pcg64 &B = e->p64;
+        TRY(e->alloc((void **)&B.z, sizeof(double) * cells));
+        TRY(e->alloc((void **)&B.op, sizeof(uint32_t) * cells));
+        TRY(e->alloc((void **)&B.words, sizeof(unsigned long long) * P64_WORDS * n));
+        TRY(e->alloc((void **)&B.blk_film, sizeof(int) * blk_film.size()));
+        CK(cudaMemcpy((void *)B.blk_film, blk_film.data(), sizeof(int) * blk_film.size(), cudaMemcpyHostToDevice));
+        TRY(e->alloc((void **)&B.err, sizeof(int)));
+        e->cg.err = B.err;
+        // as for the FP32 persistent solver: shorter waits and a block that
+        // never publishes, for the host test of the timeout
+        const char *sl = getenv("CMSL_PCG_SPIN_LIMIT"), *hb = getenv("CMSL_PCG_HOLD_BLOCK");
+        B.spin_limit = sl && atoll(sl) > 0 ? (unsigned long long)atoll(sl) : P64_SPIN_LIMIT;
+        B.hold_block = hb ? atoi(hb) : -1;
+    }
     if (e->persistent) {
         // persistent single-reduction PCG: r (the shared r), u, w, s; x =
         // correction, p in place
@@ -1649,6 +1808,7 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
     const Dev d = e->dev(0);
     if (e->precision == CMSL_FP64) k_dinv<double><<<(int)e->items.size(), NT>>>(d, (double *)e->d_dinv);
     else k_dinv<float><<<(int)e->items.size(), NT>>>(d, (float *)e->d_dinv);
+    if (e->pcg64) k_op64<<<(int)e->items.size(), NT>>>(d, (uint32_t *)e->p64.op);
     CK(cudaGetLastError());
     CK(cudaDeviceSynchronize());
     return CMSL_OK;
@@ -1888,8 +2048,7 @@ cmsl_status get_iters(Engine *e, int film, int n, int32_t *iters, int32_t *refin
 }
 
 // ms[0] TDGL, ms[1] solve set-up / first refinement pass, ms[2] and ms[3] the
-// PCG kernels (persistent FP32 solver: ms[2] per iteration, ms[3] the step
-// end; direct solve: ms[2] the solve, ms[3] the update pass, 0 under
+// PCG kernels (persistent solvers: ms[2] per iteration, ms[3] the step end; direct solve: ms[2] the solve, ms[3] the update pass, 0 under
 // deferred checks, whose TDGL kernel forms the check and is timed with every
 // depolarised film pending).  The kernels run in force mode, which leaves the
 // solver state as it is, so every repetition times the same kind of pass; the
@@ -1947,7 +2106,10 @@ cmsl_status time_kernels(Engine *e, int reps, void *stream, double *ms)
                 else TRY(launch_refine(e, st, d, F32));
                 break;
             case 2:
-                if (fp64) {
+                if (fp64 && e->pcg64) {
+                    CK(cudaMemsetAsync(e->p64.words, 0, sizeof(unsigned long long) * P64_WORDS * F, st));
+                    TRY(launch_pcg64(e, st, d, F64));      // one solve of CG_TIMING_ITERS iterations
+                } else if (fp64) {
                     k_spmv<double, Exact><<<nit, NT, 0, st>>>(d, F64);
                 } else if (e->spectral) {
                     TRY(spec_launch(e, st, d, F32));
@@ -1965,7 +2127,8 @@ cmsl_status time_kernels(Engine *e, int reps, void *stream, double *ms)
                 }
                 break;
             default:
-                if (fp64) k_update<double, Exact, false><<<nit, NT, 0, st>>>(d, F64);
+                if (fp64 && e->pcg64) k_step_end<<<1, 32, 0, st>>>(d);                   // no fourth kernel
+                else if (fp64) k_update<double, Exact, false><<<nit, NT, 0, st>>>(d, F64);
                 else if (e->spectral) TRY(launch_refine(e, st, d, F32));                 // update pass
                 else if (e->persistent) k_step_end<<<1, 32, 0, st>>>(d);                 // no fourth kernel
                 else k_update<float, Fast, true><<<nit, NT, 0, st>>>(d, F32);
@@ -1978,7 +2141,7 @@ cmsl_status time_kernels(Engine *e, int reps, void *stream, double *ms)
         float t = 0.f;
         CK(cudaEventElapsedTime(&t, a, b));
         ms[kind] = (double)t / reps;
-        if (kind == 2 && !fp64 && e->persistent) ms[kind] /= CG_TIMING_ITERS;
+        if (kind == 2 && (e->persistent || e->pcg64)) ms[kind] /= CG_TIMING_ITERS;
         CK(cudaMemcpy(e->d_solve, S.data(), sizeof(SolveDev) * F, cudaMemcpyHostToDevice));
     }
     cudaEventDestroy(a);

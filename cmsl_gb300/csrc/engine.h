@@ -7,6 +7,7 @@
 
 #include "cmsl.h"
 #include "kernels.cuh"
+#include "pcg64.cuh"
 #include "pcg_persist.cuh"
 #include "spectral.cuh"
 #include "stencil32.cuh"
@@ -150,6 +151,14 @@ struct Engine {
     void *cg_fn = nullptr;
     size_t cg_smem = 0;
 
+    // CMSL_FP64: the PCG as one cooperative launch (pcg64.cuh), or the
+    // two-kernel loop (more films than one launch carries, or
+    // CMSL_PCG_TWO_KERNEL=1)
+    bool pcg64 = false;
+    Pcg64 p64{};
+    int p64_grid = 0;
+    bool p64_resident = false;          // every film's vectors fit the warps' registers (k_pcg64r)
+
     // element stride of one P field in its set: FP32 fields are halves of float2 pairs
     int pstride() const { return precision == CMSL_FP64 ? 1 : 2; }
 
@@ -194,7 +203,8 @@ struct Engine {
         d.iters_log = d_iters; d.refine_log = d_refine;
         d.wstride = wstride; d.rstride = rstride;
         d.use_cond = use_cond; d.h_inner = hi; d.h_outer = ho;
-        d.arrive = cg.arrive;
+        if (precision == CMSL_FP64) d.words = p64.words;
+        else d.arrive = cg.arrive;
         d.maps = d_maps;
         d.err = d_err;
         return d;
@@ -223,6 +233,7 @@ cmsl_status add_kernel(cudaGraph_t g, cudaGraphNode_t *node, const cudaGraphNode
                        int grid, int block, void **args, size_t smem = 0);
 cmsl_status add_while(cudaGraph_t g, cudaGraphNode_t *node, const cudaGraphNode_t *dep, int ndep,
                       cudaGraphConditionalHandle h, cudaGraph_t *body);
+cmsl_status add_pcg64(cudaGraph_t g, cudaGraphNode_t *node, const cudaGraphNode_t *dep, const Engine *e, Dev d);
 cmsl_status build_graph(Engine *e);
 
 }  // namespace cmsl_eng

@@ -729,6 +729,8 @@ __device__ __forceinline__ void start_solves(const Dev &d, double (*sRed)[3], do
                 any |= S->active;
             }
         }
+        if (d.words)            // the persistent PCG's all-reduces start from zero
+            for (int q = threadIdx.x; q < P64_WORDS; q += blockDim.x) d.words[P64_WORDS * fi + q] = 0ull;
     }
     if (threadIdx.x == 0) {
         set_cond(d, d.h_inner, any);

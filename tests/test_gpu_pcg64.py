@@ -1,0 +1,116 @@
+"""The persistent FP64 PCG (pcg64.cuh) against the oracle's PCG of the same
+algorithm and stop test: both forms (vectors resident in registers, and
+streaming through memory, CMSL_P64_STREAM=1) at the edges of their units --
+x tiles of 32 (whole, one over, one column), rows groups of 1, 2 and 4 with
+remainders, z chunks with remainders, periodic sides shorter than a halo --
+with both z boundaries and stop tests.  Same iteration count to one and the
+potential to 1e-10 of its maximum, the tolerance of the FP64 PCG elsewhere
+(only the order and the rounding of sums differ)."""
+import os
+
+import numpy as np
+import pytest
+
+import oracle
+from tests.films import MATS_DEFAULT, random_film
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def gpu():
+    import torch
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from cmsl_gb300 import build
+    build.build()
+    import cmsl_gb300
+    return cmsl_gb300
+
+
+@pytest.mark.parametrize("zbc", [oracle.DIRICHLET, oracle.NEUMANN])
+@pytest.mark.parametrize("form", ["resident", "streaming"])
+@pytest.mark.parametrize("shape", [(1, 1, 3), (3, 2, 4), (31, 5, 3), (32, 7, 5), (33, 4, 6), (64, 3, 17), (65, 33, 9),
+                                   (96, 50, 21), (40, 130, 10)])
+def test_pcg64_solve_vs_oracle(gpu, shape, form, zbc, monkeypatch):
+    monkeypatch.setenv("CMSL_P64_STREAM", "1" if form == "streaming" else "0")
+    f, P = random_film(*shape, seed=sum(shape), zbc=zbc, eps_0_nd=3.0, layered=shape[2] >= 4,
+                       n_grains=max(2, shape[0] * shape[1] // 24))
+    if zbc == oracle.NEUMANN and shape[0] * shape[1] * shape[2] > 20000:
+        pytest.skip("the pinned operator's thousands of iterations amplify the rounding of sums beyond the tolerance")
+    if sum(shape) % 2:
+        f.tol_abs, f.tol_rel = 1e-10, 1e-8
+    else:
+        f.crit, f.tol_rel = oracle.CRIT_RELRES, 1e-9
+    f.max_iter = 4000
+    phi0 = np.random.default_rng(1).normal(size=f.N) * 1e-3     # warm start, also on the identity rows
+    want, _, _, info = oracle.load().depol_field(f, P[:3], phi0)
+    with gpu.Film.from_oracle_film(f) as g:
+        g.set_state(P, phi0)
+        res = g.depol()
+        _, phi = g.get_state()
+    if info["status"] or info["iters"] == f.max_iter:
+        return                  # no solve: a start on the identity rows makes the 3-cell film's system non-symmetric
+    assert res["status"] == 0
+    assert abs(res["iters"] - info["iters"]) <= 1
+    if res["iters"] == info["iters"]:
+        assert np.abs(phi - want).max() <= 1e-10 * np.abs(want).max()
+    else:                                                       # one iteration apart: the stop test's own accuracy
+        assert np.abs(phi - want).max() <= 1e-6 * np.abs(want).max()
+
+
+def test_pcg64_film_beyond_the_resident_form(gpu):
+    """A film of more units than warps takes the streaming form by itself (z
+    chunks and rows as its plan picks them)."""
+    mats = MATS_DEFAULT.copy()
+    mats[:, 7] = 30.0
+    f, P = random_film(100, 96, 60, seed=9, eps_0_nd=3.0, mats=mats)
+    f.crit, f.tol_rel, f.max_iter = oracle.CRIT_RELRES, 1e-9, 4000
+    want, _, _, info = oracle.load().depol_field(f, P[:3], np.zeros(f.N))
+    with gpu.Film.from_oracle_film(f) as g:
+        g.set_state(P)
+        res = g.depol()
+        _, phi = g.get_state()
+    assert res["status"] == 0 and abs(res["iters"] - info["iters"]) <= 1
+    assert np.abs(phi - want).max() <= (1e-10 if res["iters"] == info["iters"] else 1e-6) * np.abs(want).max()
+
+
+def test_pcg64_iteration_cap_and_two_kernel_form(gpu, monkeypatch):
+    """A solve that ends on its iteration cap, and the two-kernel loop
+    (CMSL_PCG_TWO_KERNEL=1), give the same iterate."""
+    f, P = random_film(48, 20, 8, seed=5, eps_0_nd=3.0)
+    f.crit, f.tol_rel, f.max_iter = oracle.CRIT_RELRES, 1e-12, 7
+    out = []
+    for two in ("0", "1"):
+        monkeypatch.setenv("CMSL_PCG_TWO_KERNEL", two)
+        with gpu.Film.from_oracle_film(f) as g:
+            g.set_state(P)
+            assert g.depol()["iters"] == 7
+            out.append(g.get_state()[1])
+    assert np.abs(out[0] - out[1]).max() <= 1e-12 * np.abs(out[1]).max()
+
+
+def test_pcg64_wait_timeout_is_reported(gpu):
+    """A block that never adds its sums (held back on the host at creation,
+    with short waits): every wait runs out, the kernel returns, the run
+    reports CMSL_ERR_CUDA and the context stays usable."""
+    f, P = random_film(64, 32, 8, seed=71, eps_0_nd=3.0, p_scale=0.2)
+    keys = {"CMSL_PCG_HOLD_BLOCK": "1", "CMSL_PCG_SPIN_LIMIT": "2000"}
+    old = {k: os.environ.get(k) for k in keys}
+    os.environ.update(keys)
+    try:
+        g = gpu.Film.from_oracle_film(f)
+    finally:
+        for k, v in old.items():
+            os.environ.pop(k) if v is None else os.environ.__setitem__(k, v)
+    try:
+        g.set_state(P)
+        with pytest.raises(gpu.CmslError) as e:
+            g.run(np.full(2, 0.1))
+        assert e.value.status == 2 and "barrier timed out" in str(e.value)
+    finally:
+        g.close()
+    with gpu.Film.from_oracle_film(f) as h:
+        h.set_state(P)
+        h.run(np.full(2, 0.1))
+        assert all(np.isfinite(p).all() for p in h.get_state()[0])
