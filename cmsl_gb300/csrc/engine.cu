@@ -30,6 +30,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <functional>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -189,8 +190,26 @@ SpecAxis spec_plan(int n)
     SpecAxis a{};
     a.n = n;
     a.lg = (n & (n - 1)) == 0 ? __builtin_ctz((unsigned)n) : -1;
-    while (n % 3 == 0) { a.rad[a.nst++] = 3; n /= 3; }
-    while (n % 2 == 0) { a.rad[a.nst++] = 2; n /= 2; }
+    if (a.lg >= 0) return a;
+    // the fewest passes; the radices as even as they can be (the least largest
+    // one), so that every pass has butterflies for most threads
+    static const int R[] = {16, 12, 9, 8, 6, 4, 3, 2};
+    std::vector<int> best, cur;
+    std::function<void(int, int)> go = [&](int m, int from) {
+        if (m == 1) {
+            if (best.empty() || cur.size() < best.size() || (cur.size() == best.size() && cur[0] < best[0])) best = cur;
+            return;
+        }
+        if (!best.empty() && cur.size() >= best.size()) return;
+        for (int i = from; i < 8; ++i)
+            if (m % R[i] == 0) {
+                cur.push_back(R[i]);
+                go(m / R[i], i);
+                cur.pop_back();
+            }
+    };
+    go(n, 0);
+    for (int r : best) a.rad[a.nst++] = r;
     return a;
 }
 
@@ -496,15 +515,15 @@ cmsl_status build_graph(Engine *e)
         }
         struct Node { void *fn; int grid, block; void **args; size_t smem; };
         const Node rows[] = {
-            {(void *)k_spec_x<true>, e->spec_grid[0], SPEC_NT, a_x, e->spec_smem[0]},
-            {(void *)k_spec_y, e->spec_grid[1], SPEC_NT, a_s, e->spec_smem[1]},
+            {e->spec_x[0], e->spec_grid[0], SPEC_NT, a_x, e->spec_smem[0]},
+            {e->spec_y, e->spec_grid[1], SPEC_NT, a_s, e->spec_smem[1]},
             {(void *)k_spec_z<false>, e->spec_grid[2], e->spec_zt, a_s, e->spec_smem[2]},
-            {(void *)k_spec_y, e->spec_grid[1], SPEC_NT, a_s, e->spec_smem[1]},
-            {(void *)k_spec_x<false>, e->spec_grid[0], SPEC_NT, a_x, e->spec_smem[0]}};
+            {e->spec_y, e->spec_grid[1], SPEC_NT, a_s, e->spec_smem[1]},
+            {e->spec_x[1], e->spec_grid[0], SPEC_NT, a_x, e->spec_smem[0]}};
         const Node cols[] = {
-            {(void *)k_spec_x<true, true>, e->spec_grid[0], SPEC_NT, a_x, e->spec_smem[0]},
-            {(void *)k_spec_yzy, e->spec_grid[3], SPEC_YZY_NT, a_s, e->spec_smem[3]},
-            {(void *)k_spec_x<false, true>, e->spec_grid[0], SPEC_NT, a_x, e->spec_smem[0]}};
+            {e->spec_x[0], e->spec_grid[0], SPEC_NT, a_x, e->spec_smem[0]},
+            {e->spec_yzy, e->spec_grid[3], SPEC_YZY_NT, a_s, e->spec_smem[3]},
+            {e->spec_x[1], e->spec_grid[0], SPEC_NT, a_x, e->spec_smem[0]}};
         const Node clus[] = {
             {(void *)k_spec_cxy, e->spec_grid[4], SPEC_CL_NT, a_x, e->spec_smem[4]},
             {(void *)k_spec_z<true>, e->spec_grid[2], e->spec_zt, a_s, e->spec_smem[2]},
@@ -843,19 +862,22 @@ cmsl_status spec_launch(Engine *e, cudaStream_t st, const Dev &d, const Fields<f
         CK(cudaGetLastError());
         return CMSL_OK;
     }
+    Dev dd = d;
+    Fields<float> ff = F32;
+    SpecDev ss = sp;
+    void *a_x[] = {&dd, &ff, &ss}, *a_s[] = {&dd, &ss};
+    auto go = [&](void *fn, int grid, int block, void **args, size_t smem) {
+        return cudaLaunchKernel(fn, dim3((unsigned)grid), dim3((unsigned)block), args, smem, st);
+    };
+    CK(go(e->spec_x[0], e->spec_grid[0], SPEC_NT, a_x, e->spec_smem[0]));
     if (e->spec_col) {
-        k_spec_x<true, true><<<e->spec_grid[0], SPEC_NT, e->spec_smem[0], st>>>(d, F32, sp);
-        k_spec_yzy<<<e->spec_grid[3], SPEC_YZY_NT, e->spec_smem[3], st>>>(d, sp);
-        k_spec_x<false, true><<<e->spec_grid[0], SPEC_NT, e->spec_smem[0], st>>>(d, F32, sp);
-        CK(cudaGetLastError());
-        return CMSL_OK;
+        CK(go(e->spec_yzy, e->spec_grid[3], SPEC_YZY_NT, a_s, e->spec_smem[3]));
+    } else {
+        CK(go(e->spec_y, e->spec_grid[1], SPEC_NT, a_s, e->spec_smem[1]));
+        CK(go((void *)k_spec_z<false>, e->spec_grid[2], e->spec_zt, a_s, e->spec_smem[2]));
+        CK(go(e->spec_y, e->spec_grid[1], SPEC_NT, a_s, e->spec_smem[1]));
     }
-    k_spec_x<true><<<e->spec_grid[0], SPEC_NT, e->spec_smem[0], st>>>(d, F32, sp);
-    k_spec_y<<<e->spec_grid[1], SPEC_NT, e->spec_smem[1], st>>>(d, sp);
-    k_spec_z<false><<<e->spec_grid[2], e->spec_zt, e->spec_smem[2], st>>>(d, sp);
-    k_spec_y<<<e->spec_grid[1], SPEC_NT, e->spec_smem[1], st>>>(d, sp);
-    k_spec_x<false><<<e->spec_grid[0], SPEC_NT, e->spec_smem[0], st>>>(d, F32, sp);
-    CK(cudaGetLastError());
+    CK(go(e->spec_x[1], e->spec_grid[0], SPEC_NT, a_x, e->spec_smem[0]));
     return CMSL_OK;
 }
 
@@ -1672,9 +1694,23 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
         e->spec_smem[0] = smx;
         e->spec_smem[1] = smy;
         e->spec_smem[2] = spec_zbytes(spec_mmax) * zt;
-        CK(cudaFuncSetAttribute(k_spec_x<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e->spec_smem[0]));
-        CK(cudaFuncSetAttribute(k_spec_x<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e->spec_smem[0]));
-        CK(cudaFuncSetAttribute(k_spec_y, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e->spec_smem[1]));
+        {
+            bool mixed = false;
+            for (int fi = 0; fi < n; ++fi) mixed |= e->fh[fi].dep && (sf[fi].ax.lg < 0 || sf[fi].ay.lg < 0);
+            const bool col = e->spec_col && !e->spec_cl;
+            e->spec_x[0] = col ? mixed ? (void *)k_spec_x<true, true, true> : (void *)k_spec_x<true, true, false>
+                               : mixed ? (void *)k_spec_x<true, false, true> : (void *)k_spec_x<true, false, false>;
+            e->spec_x[1] = col ? mixed ? (void *)k_spec_x<false, true, true> : (void *)k_spec_x<false, true, false>
+                               : mixed ? (void *)k_spec_x<false, false, true> : (void *)k_spec_x<false, false, false>;
+            e->spec_y = mixed ? (void *)k_spec_y<true> : (void *)k_spec_y<false>;
+            e->spec_yzy = mixed ? (void *)k_spec_yzy<true> : (void *)k_spec_yzy<false>;
+            e->spec_grid[3] = (int)bqf.size();
+            e->spec_smem[3] = smq;
+            for (void *fn : e->spec_x)
+                CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e->spec_smem[0]));
+            CK(cudaFuncSetAttribute(e->spec_y, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e->spec_smem[1]));
+            if (col) CK(cudaFuncSetAttribute(e->spec_yzy, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smq));
+        }
         CK(cudaFuncSetAttribute(k_spec_z<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e->spec_smem[2]));
         CK(cudaFuncSetAttribute(k_spec_z<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e->spec_smem[2]));
         if (e->spec_cl) {
@@ -1682,17 +1718,6 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
             e->spec_smem[4] = smc;
             CK(cudaFuncSetAttribute(k_spec_cxy, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smc));
             CK(cudaFuncSetAttribute(k_spec_cyx, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smc));
-        }
-        {
-            e->spec_grid[3] = (int)bqf.size();
-            e->spec_smem[3] = smq;
-            if (e->spec_col && !e->spec_cl) {
-                CK(cudaFuncSetAttribute(k_spec_x<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)e->spec_smem[0]));
-                CK(cudaFuncSetAttribute(k_spec_x<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)e->spec_smem[0]));
-                CK(cudaFuncSetAttribute(k_spec_yzy, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smq));
-            }
         }
     }
     TRY(e->alloc((void **)&e->d_phi[0], sizeof(double) * cells));

@@ -101,6 +101,7 @@ struct Engine {
     int refine_nt = 0, tdgl_nt = 0;     // threads per block
     bool spectral = false;      // FP32 inner solve by the direct spectral solve (one film, uniform eps)
     SpecDev spec{};
+    void *spec_x[2] = {nullptr, nullptr}, *spec_y = nullptr, *spec_yzy = nullptr;   // x forward and inverse, y, y-z-y
     int spec_grid[5] = {0, 0, 0, 0, 0};   // blocks of the x, y, z passes, the column-pair pass, the cluster passes
     int spec_zt = 0;            // threads per block of the z solve
     size_t spec_smem[5] = {0, 0, 0, 0, 0};

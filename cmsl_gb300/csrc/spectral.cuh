@@ -20,7 +20,7 @@
 //
 // FFTs: self-sorting (Stockham) passes through shared memory, the butterflies
 // in registers -- radix 16 (8, 4 or 2 for the remainder) for powers of two,
-// radix 3 and 2 otherwise -- one block per group of rows (x) or of columns
+// the fewest radices up to 16 otherwise -- one block per group of rows (x) or of columns
 // (y); twiddles exp(-2 pi i t / n) and eigenvalues come from host tables
 // computed in double.  The z solve keeps the Thomas elimination in shared
 // memory, so each spectrum value is read and written once per sweep.
@@ -257,50 +257,146 @@ __device__ __forceinline__ void fft_pow2(float2 *a, float2 *b, int nseq, int lgn
     }
 }
 
-// Any 2^a 3^b length: radix-3 and radix-2 passes.
-template <bool SEQ_FAST>
-__device__ __forceinline__ float2 *fft_mixed(float2 *a, float2 *b, int nseq, const SpecAxis &pl, int es, int ss,
-                                             const float2 *tw)
+// Forward DFTs of 3, 6, 9 and 12 values in registers, natural order: 6 and 12
+// by the prime-factor map (2 x 3, 4 x 3: no twiddles), 9 as 3 x 3.
+__device__ __forceinline__ void dft3(float2 &a, float2 &b, float2 &c)
 {
-    const int n = pl.n;
-    int Ns = 1;
-    for (int st = 0; st < pl.nst; ++st) {
-        const int R = pl.rad[st];
-        const int nbf = n / R;
-        const int tstride = n / (Ns * R);
-        for (int t = threadIdx.x; t < nseq * nbf; t += blockDim.x) {
-            int sq, j;
-            if (SEQ_FAST) { j = t / nseq; sq = t - j * nseq; }
-            else { sq = t / nbf; j = t - sq * nbf; }
-            const int jm = j % Ns;
-            const int base = sq * ss;
-            auto at = [&](int e) { return SEQ_FAST ? base + e * es : spec_pad(base + e * es); };
-            const int o = (j / Ns) * Ns * R + jm;
-            const float2 v0 = a[at(j)];
-            const float2 v1 = c_mul(a[at(j + nbf)], tw[jm * tstride]);
-            if (R == 2) {
-                b[at(o)] = c_add(v0, v1);
-                b[at(o + Ns)] = c_sub(v0, v1);
-            } else {
-                const float2 v2 = c_mul(a[at(j + 2 * nbf)], tw[2 * jm * tstride]);
-                const float2 s12 = c_add(v1, v2), d12 = c_sub(v1, v2);
-                const float2 m = make_float2(v0.x - 0.5f * s12.x, v0.y - 0.5f * s12.y);
-                const float k3 = 0.86602540378443865f;   // sin(2 pi / 3)
-                const float2 rot = make_float2(k3 * d12.y, -k3 * d12.x);
-                b[at(o)] = c_add(v0, s12);
-                b[at(o + Ns)] = c_add(m, rot);
-                b[at(o + 2 * Ns)] = c_sub(m, rot);
-            }
+    const float k3 = 0.86602540378443865f;             // sin(2 pi / 3)
+    const float2 s = c_add(b, c), d = c_sub(b, c);
+    const float2 m = make_float2(a.x - 0.5f * s.x, a.y - 0.5f * s.y), rot = make_float2(k3 * d.y, -k3 * d.x);
+    a = c_add(a, s);
+    b = c_add(m, rot);
+    c = c_sub(m, rot);
+}
+__device__ __forceinline__ void dft6(float2 (&v)[6])
+{
+    // n = 3 n1 + 2 n2, k = 3 k1 + 4 k2 (mod 6)
+    float2 a0 = v[0], a1 = v[2], a2 = v[4], b0 = v[3], b1 = v[5], b2 = v[1];
+    dft3(a0, a1, a2);
+    dft3(b0, b1, b2);
+    v[0] = c_add(a0, b0); v[3] = c_sub(a0, b0);
+    v[4] = c_add(a1, b1); v[1] = c_sub(a1, b1);
+    v[2] = c_add(a2, b2); v[5] = c_sub(a2, b2);
+}
+__device__ __forceinline__ void dft12(float2 (&v)[12])
+{
+    // n = 3 n1 + 4 n2, k = 9 k1 + 4 k2 (mod 12)
+    float2 t[3][4];
+    #pragma unroll
+    for (int n2 = 0; n2 < 3; ++n2) {
+        #pragma unroll
+        for (int n1 = 0; n1 < 4; ++n1) t[n2][n1] = v[(3 * n1 + 4 * n2) % 12];
+        dft4(t[n2][0], t[n2][1], t[n2][2], t[n2][3]);
+    }
+    #pragma unroll
+    for (int k1 = 0; k1 < 4; ++k1) {
+        dft3(t[0][k1], t[1][k1], t[2][k1]);
+        #pragma unroll
+        for (int k2 = 0; k2 < 3; ++k2) v[(9 * k1 + 4 * k2) % 12] = t[k2][k1];
+    }
+}
+// v exp(-2 pi i e / 9) for the exponents n2 k1 (1, 2, 4) of the 3 x 3 split
+__device__ __forceinline__ float2 w9(int e, float2 v)
+{
+    return e == 1 ? c_mulc(v, 0.76604444311897804f, -0.64278760968653933f)
+         : e == 2 ? c_mulc(v, 0.17364817766693035f, -0.98480775301220806f)
+                  : c_mulc(v, -0.93969262078590838f, -0.34202014332566873f);
+}
+__device__ __forceinline__ void dft9(float2 (&v)[9])
+{
+    // n = 3 n1 + n2, k = k1 + 3 k2: DFT3 over n1, twiddle w9^(n2 k1), DFT3 over n2
+    #pragma unroll
+    for (int n2 = 0; n2 < 3; ++n2) dft3(v[n2], v[3 + n2], v[6 + n2]);
+    #pragma unroll
+    for (int k1 = 1; k1 < 3; ++k1)
+        #pragma unroll
+        for (int n2 = 1; n2 < 3; ++n2) v[3 * k1 + n2] = w9(n2 * k1, v[3 * k1 + n2]);
+    #pragma unroll
+    for (int k1 = 0; k1 < 3; ++k1) dft3(v[3 * k1], v[3 * k1 + 1], v[3 * k1 + 2]);
+}
+
+// Quotients by a divisor d of the pass (x d < 2^32): one high multiply.
+struct FastDiv {
+    unsigned int d, m;
+    __device__ __forceinline__ explicit FastDiv(int div) : d((unsigned)div), m(div > 1 ? 0xffffffffu / (unsigned)div + 1u : 0u) {}
+    __device__ __forceinline__ int quo(int x) const { return d > 1u ? (int)__umulhi((unsigned)x, m) : x; }
+};
+
+// A Stockham pass (as stockham_pass) of any radix at any Ns.
+template <int R, bool SEQ_FAST, class LD, class ST>
+__device__ __forceinline__ void stockham_mixed(const float2 *a, float2 *b, int nseq, int n, int Ns, int es, int ss,
+                                               const float2 *tw, bool first, bool last, LD &ld, ST &st)
+{
+    const int nbf = n / R, step = nbf / Ns, total = nseq * nbf;
+    const FastDiv fq(SEQ_FAST ? nseq : nbf), fn(Ns);
+    for (int t = threadIdx.x; t < total; t += blockDim.x) {
+        const int q = fq.quo(t);
+        const int sq = SEQ_FAST ? t - q * nseq : q, j = SEQ_FAST ? q : t - q * nbf;
+        const int jq = fn.quo(j), jm = j - jq * Ns;
+        const int o = jq * Ns * R + jm, base = sq * ss, tj = jm * step;
+        auto at = [&](int e) { return SEQ_FAST ? base + e * es : spec_pad(base + e * es); };
+        float2 v[R];
+        #pragma unroll
+        for (int r = 0; r < R; ++r) v[r] = first ? ld(sq, j + r * nbf) : a[at(j + r * nbf)];
+        if (Ns > 1) {
+            #pragma unroll
+            for (int r = 1; r < R; ++r) v[r] = c_mul(v[r], tw[r * tj]);
         }
-        __syncthreads();
+        if constexpr (R == 3) dft3(v[0], v[1], v[2]);
+        else if constexpr (R == 6) dft6(v);
+        else if constexpr (R == 9) dft9(v);
+        else if constexpr (R == 12) dft12(v);
+        else dft_reg<R>(v);
+        #pragma unroll
+        for (int i = 0; i < R; ++i) {
+            const int k = R == 9 ? (i / 3) + 3 * (i % 3) : dft_out<R>(i);
+            if (last) st(sq, o + k * Ns, v[i]);
+            else b[at(o + k * Ns)] = v[i];
+        }
+    }
+}
+
+// Lengths 2^a 3^b that are no power of two: the passes of pl (spec_plan: the
+// fewest radices of 16, 12, 9, 8, 6, 4, 3, 2 whose product is n -- 96 = 16 x 6
+// and 192 = 16 x 12 take two), between ld and st as fft_pow2.  One radix-2 or
+// -3 pass through shared memory per factor took 6 to 7 passes: the solve of a
+// 192x96x24 film 56 us, now 33.
+template <bool SEQ_FAST, class LD, class ST>
+__device__ __forceinline__ void fft_mixed(float2 *a, float2 *b, int nseq, const SpecAxis &pl, int es, int ss,
+                                          const float2 *tw, LD ld, ST st)
+{
+    int Ns = 1;
+    for (int q = 0; q < pl.nst; ++q) {
+        const int R = pl.rad[q];
+        const bool first = q == 0, last = q + 1 == pl.nst;
+        switch (R) {
+        case 16: stockham_mixed<16, SEQ_FAST>(a, b, nseq, pl.n, Ns, es, ss, tw, first, last, ld, st); break;
+        case 12: stockham_mixed<12, SEQ_FAST>(a, b, nseq, pl.n, Ns, es, ss, tw, first, last, ld, st); break;
+        case 9: stockham_mixed<9, SEQ_FAST>(a, b, nseq, pl.n, Ns, es, ss, tw, first, last, ld, st); break;
+        case 8: stockham_mixed<8, SEQ_FAST>(a, b, nseq, pl.n, Ns, es, ss, tw, first, last, ld, st); break;
+        case 6: stockham_mixed<6, SEQ_FAST>(a, b, nseq, pl.n, Ns, es, ss, tw, first, last, ld, st); break;
+        case 4: stockham_mixed<4, SEQ_FAST>(a, b, nseq, pl.n, Ns, es, ss, tw, first, last, ld, st); break;
+        case 3: stockham_mixed<3, SEQ_FAST>(a, b, nseq, pl.n, Ns, es, ss, tw, first, last, ld, st); break;
+        default: stockham_mixed<2, SEQ_FAST>(a, b, nseq, pl.n, Ns, es, ss, tw, first, last, ld, st); break;
+        }
+        if (!last) __syncthreads();
         float2 *tmp = a;
         a = b;
         b = tmp;
         Ns *= R;
     }
-    return a;
 }
 
+// The transform of nseq sequences along ax between ld and st.  MIXED: the
+// launch has films whose sides are no powers of two (a compile-time choice:
+// the radices of those cost the others' kernels registers).
+template <bool SEQ_FAST, bool MIXED, class LD, class ST>
+__device__ __forceinline__ void fft_any(float2 *a, float2 *b, int nseq, const SpecAxis &ax, int es, int ss,
+                                        const float2 *tw, LD ld, ST st)
+{
+    if (!MIXED || ax.lg >= 0) fft_pow2<SEQ_FAST>(a, b, nseq, ax.lg, es, ss, tw, ld, st);
+    else if constexpr (MIXED) fft_mixed<SEQ_FAST>(a, b, nseq, ax, es, ss, tw, ld, st);
+}
 
 // Whether film f's inner solve runs through the spectra in this pass.
 __device__ __forceinline__ bool spec_run(const Dev &d, int f)
@@ -354,7 +450,12 @@ __device__ __forceinline__ int fft_pow2_passes(int lgn)
     return n;
 }
 
-template <bool IN_REAL, bool COL = false>
+template <bool MIXED> __device__ __forceinline__ int fft_passes(const SpecAxis &ax)
+{
+    return !MIXED || ax.lg >= 0 ? fft_pow2_passes(ax.lg) : ax.nst;
+}
+
+template <bool IN_REAL, bool COL, bool MIXED>
 __global__ void __launch_bounds__(SPEC_NT, 4) k_spec_x(Dev d, Fields<float> F, SpecDev sp)
 {
     extern __shared__ float2 sm2[];
@@ -370,7 +471,7 @@ __global__ void __launch_bounds__(SPEC_NT, 4) k_spec_x(Dev d, Fields<float> F, S
     const float *rr = F.r + P.off;
     float *xx = F.x + P.off;
     float2 *Cf = sp.C + P.coff;
-    const SpecAxis ax = P.ax;
+    const SpecAxis &ax = P.ax;
     const int M = P.M, Mp = P.Mp;
     // row pitch of the tiles: nx, or nx + 1 in the column layout, whose
     // transposed copies read a column of the tile (an odd pitch in 8-byte
@@ -402,7 +503,7 @@ __global__ void __launch_bounds__(SPEC_NT, 4) k_spec_x(Dev d, Fields<float> F, S
         return make_float2(rr[o], 2 * j + 1 < M ? rr[o + plane] : 0.f);
     };
     // the tile that receives the transform in the column layout's store
-    float2 *res = (ax.lg >= 0 && (fft_pow2_passes(ax.lg) & 1) == 0) ? a : b;
+    float2 *res = (fft_passes<MIXED>(ax) & 1) == 0 ? a : b;
     // the increment of this solve: w M^-1 r + m (the previous increment), from
     // the film's Chebyshev recurrence (w = 1, m = 0 for an exact solve)
     const SolveDev *Sf = d.solve + f;
@@ -427,24 +528,8 @@ __global__ void __launch_bounds__(SPEC_NT, 4) k_spec_x(Dev d, Fields<float> F, S
         if (j == 0) xx[yx] = 0.f;                                        // first Dirichlet plane
         if (j == Mp - 1) xx[(long long)(M + 1) * plane + yx] = 0.f;      // last one
     };
-    if (ax.lg >= 0) {
-        __syncthreads();                                                 // twiddles
-        fft_pow2<false>(a, b, nr, ax.lg, 1, pitch, tw, ld, st);
-    } else {
-        const int total = nr * nx;
-        if (!(COL && !IN_REAL))
-            for (int t = threadIdx.x; t < total; t += blockDim.x) {
-                const int sq = t / nx, e = t - sq * nx;
-                a[spec_pad(sq * pitch + e)] = ld(sq, e);
-            }
-        __syncthreads();
-        res = fft_mixed<false>(a, b, nr, ax, 1, pitch, tw);
-        if (!(COL && IN_REAL))
-            for (int t = threadIdx.x; t < total; t += blockDim.x) {
-                const int sq = t / nx, e = t - sq * nx;
-                st(sq, e, res[spec_pad(sq * pitch + e)]);
-            }
-    }
+    __syncthreads();                                                     // twiddles
+    fft_any<false, MIXED>(a, b, nr, ax, 1, pitch, tw, ld, st);
     if (COL && IN_REAL) {
         // transposed store: consecutive threads write consecutive rows of one column
         __syncthreads();
@@ -459,7 +544,7 @@ __global__ void __launch_bounds__(SPEC_NT, 4) k_spec_x(Dev d, Fields<float> F, S
 
 // y transforms of column groups of one packed plane, in place on the
 // spectra; the tile keeps the plane's row-major layout (sequences interleaved).
-static __global__ void __launch_bounds__(SPEC_NT, 4) k_spec_y(Dev d, SpecDev sp)
+template <bool MIXED> __global__ void __launch_bounds__(SPEC_NT, 4) k_spec_y(Dev d, SpecDev sp)
 {
     extern __shared__ float2 sm2[];
     const int f = __ldg(sp.by_film + blockIdx.x);
@@ -469,7 +554,7 @@ static __global__ void __launch_bounds__(SPEC_NT, 4) k_spec_y(Dev d, SpecDev sp)
     const int groups = (nx + cb - 1) / cb;
     const int lb = blockIdx.x - P.by0;
     const int kk = lb / groups, x0 = (lb - kk * groups) * cb, nc = min(cb, nx - x0);
-    const SpecAxis ay = P.ay;
+    const SpecAxis &ay = P.ay;
     float2 *base = sp.C + P.coff + (long long)kk * nx * ny + x0;
     float2 *a = sm2, *b = sm2 + cb * ny, *tw = sm2 + 2 * cb * ny;
     for (int t = threadIdx.x; t < ny; t += blockDim.x) tw[t] = __ldg(sp.tw + P.twy + t);
@@ -477,15 +562,7 @@ static __global__ void __launch_bounds__(SPEC_NT, 4) k_spec_y(Dev d, SpecDev sp)
     auto ld = [&](int c, int e) { return base[(long long)e * nx + c]; };
     auto st = [&](int c, int e, float2 v) { base[(long long)e * nx + c] = v; };
     __syncthreads();                                                     // twiddles
-    if (ay.lg >= 0) {
-        fft_pow2<true>(a, b, nc, ay.lg, nc, 1, tw, ld, st);
-    } else {
-        const int total = nc * ny;
-        for (int t = threadIdx.x; t < total; t += blockDim.x) a[t] = ld(t % nc, t / nc);
-        __syncthreads();
-        const float2 *res = fft_mixed<true>(a, b, nc, ay, nc, 1, tw);
-        for (int t = threadIdx.x; t < total; t += blockDim.x) st(t % nc, t / nc, res[t]);
-    }
+    fft_any<true, MIXED>(a, b, nc, ay, nc, 1, tw, ld, st);
 }
 
 // In-plane modes m whose mirror -m has an index >= m's, one per z solve:
@@ -620,7 +697,7 @@ __host__ __device__ inline size_t spec_yzy_bytes(int ny, int Mp, int M)
 
 constexpr int SPEC_YZY_NT = 512;
 
-static __global__ void __launch_bounds__(SPEC_YZY_NT, 1) k_spec_yzy(Dev d, SpecDev sp)
+template <bool MIXED> __global__ void __launch_bounds__(SPEC_YZY_NT, 1) k_spec_yzy(Dev d, SpecDev sp)
 {
     extern __shared__ float2 sm2[];
     const int f = __ldg(sp.bq_film + blockIdx.x);
@@ -631,7 +708,7 @@ static __global__ void __launch_bounds__(SPEC_YZY_NT, 1) k_spec_yzy(Dev d, SpecD
     const int ncol = kx == kx2 ? 1 : 2, nseq = ncol * Mp;
     const int tile = spec_pad(2 * Mp * ny) + 1;
     float2 *A = sm2, *B = sm2 + tile, *tw = sm2 + 2 * tile;
-    const SpecAxis ay = P.ay;
+    const SpecAxis &ay = P.ay;
     const long long modes = (long long)nx * ny;
     float2 *Cf = sp.C + P.coff;
     auto gcol = [&](int sq) {                    // first value of sequence sq in the spectra
@@ -649,18 +726,12 @@ static __global__ void __launch_bounds__(SPEC_YZY_NT, 1) k_spec_yzy(Dev d, SpecD
     for (int t = threadIdx.x; t < ny; t += blockDim.x) tw[t] = __ldg(sp.tw + P.twy + t);
     __syncthreads();
     // forward y transforms: spectra -> tile R
-    float2 *R;
-    if (ay.lg >= 0) {
-        R = (fft_pow2_passes(ay.lg) & 1) == 0 ? A : B;
+    float2 *R = (fft_passes<MIXED>(ay) & 1) == 0 ? A : B;
+    {
         auto ld = [&](int sq, int e) { return gcol(sq)[e]; };
         auto st = [&](int sq, int e, float2 v) { R[spec_pad(sq * ny + e)] = v; };
-        fft_pow2<false>(A, B, nseq, ay.lg, 1, ny, tw, ld, st);
-    } else {
-        for (int t = threadIdx.x; t < nseq * ny; t += blockDim.x) A[spec_pad(t)] = gcol(t / ny)[t - (t / ny) * ny];
-        __syncthreads();
-        R = fft_mixed<false>(A, B, nseq, ay, 1, ny, tw);
+        fft_any<false, MIXED>(A, B, nseq, ay, 1, ny, tw, ld, st);
     }
-    __syncthreads();
     cp_wait<0>();
     __syncthreads();
     // z solve, one thread per mode pair (as k_spec_z)
@@ -718,15 +789,9 @@ static __global__ void __launch_bounds__(SPEC_YZY_NT, 1) k_spec_yzy(Dev d, SpecD
     }
     __syncthreads();
     // y transforms of the conjugated solutions: tile R -> spectra
-    if (ay.lg >= 0) {
-        float2 *other = R == A ? B : A;
-        auto ld = [&](int sq, int e) { return R[spec_pad(sq * ny + e)]; };
-        auto st = [&](int sq, int e, float2 v) { gcol(sq)[e] = v; };
-        fft_pow2<false>(R, other, nseq, ay.lg, 1, ny, tw, ld, st);
-    } else {
-        const float2 *res = fft_mixed<false>(R, R == A ? B : A, nseq, ay, 1, ny, tw);
-        for (int t = threadIdx.x; t < nseq * ny; t += blockDim.x) gcol(t / ny)[t - (t / ny) * ny] = res[spec_pad(t)];
-    }
+    auto ld = [&](int sq, int e) { return R[spec_pad(sq * ny + e)]; };
+    auto st = [&](int sq, int e, float2 v) { gcol(sq)[e] = v; };
+    fft_any<false, MIXED>(R, R == A ? B : A, nseq, ay, 1, ny, tw, ld, st);
 }
 
 // ------------------------------------------------- cluster transforms
