@@ -819,13 +819,18 @@ cmsl_status read_flags(Engine *e, cudaStream_t st, bool *active, bool *outer)
     return CMSL_OK;
 }
 
-// One FP32 residual pass (k_refine32) launched from the host.
+// One FP32 residual pass (k_refine32) launched from the host.  Where F32's
+// two P sets are pointed at one (solves of the current state), the pass takes
+// the cp.async ring: the tensor maps name the sets themselves.
 cmsl_status launch_refine(Engine *e, cudaStream_t st, const Dev &d, const Fields<float> &F32)
 {
     Dev dd = d;
     Fields<float> ff = F32;
     void *args[] = {&dd, &ff};
-    CK(cudaLaunchKernel(e->refine_fn, dim3((unsigned)e->sitems.size()), dim3(e->refine_nt), args, e->refine_smem, st));
+    const bool ring = F32.P[0][0] == F32.P[1][0];
+    const int yi = Engine::ty_index(e->stile_ty);
+    CK(cudaLaunchKernel(ring ? e->refine_cp[yi] : e->refine_fn, dim3((unsigned)e->sitems.size()), dim3(e->refine_nt), args,
+                        ring ? e->refine_cp_smem[yi] : e->refine_smem, st));
     return CMSL_OK;
 }
 
