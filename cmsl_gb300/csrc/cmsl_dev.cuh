@@ -119,6 +119,7 @@ struct SolveDev {               // per film, lives in device memory
                                 // forming b - A phi in double-float
     double cheb_rho;            // Chebyshev recurrence of the preconditioned refinement (rho_k)
     float cheb_w, cheb_m;       // the next direct solve's increment: dx <- w M^-1 r + m dx
+    float pin_r, pin_x;         // direct solve of a Neumann film: r and the previous increment at the pinned cell
     int row_pend;               // Dev::row_off: the sweep row (+1; 0 none) whose item partials the
                                 // TDGL step left for the next residual pass to total and write
     int pending;                // the step ended on its direct solve: the potential is phi_cur (the

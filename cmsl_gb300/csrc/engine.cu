@@ -530,9 +530,12 @@ cmsl_status build_graph(Engine *e)
             {(void *)k_spec_cyx, e->spec_grid[4], SPEC_CL_NT, a_x, e->spec_smem[4]}};
         const Node *seq = e->spec_cl ? clus : e->spec_col ? cols : rows;
         const int nseq = e->spec_cl || e->spec_col ? 3 : 5;
+        const Node pin = {(void *)k_spec_pin, e->spec_pin, SPEC_NT, a_x, 0};
+        const Node shift = {(void *)k_spec_shift, e->spec_pin, SPEC_NT, a_x, 0};
         const cudaGraphNode_t *prev = dep;
-        for (int qi = 0; qi < nseq; ++qi) {
-            const Node &q = seq[qi];
+        const int lead = e->spec_pin ? 1 : 0;            // Neumann films: pin, ..., shift
+        for (int qi = -lead; qi < nseq + lead; ++qi) {
+            const Node &q = qi < 0 ? pin : qi == nseq ? shift : seq[qi];
             TRY(add_kernel(gs, out, prev, prev ? 1 : 0, q.fn, q.grid, q.block, q.args, q.smem));
             prev = out;
         }
@@ -874,6 +877,7 @@ cmsl_status spec_launch(Engine *e, cudaStream_t st, const Dev &d, const Fields<f
     auto go = [&](void *fn, int grid, int block, void **args, size_t smem) {
         return cudaLaunchKernel(fn, dim3((unsigned)grid), dim3((unsigned)block), args, smem, st);
     };
+    if (e->spec_pin) CK(go((void *)k_spec_pin, e->spec_pin, SPEC_NT, a_x, 0));
     CK(go(e->spec_x[0], e->spec_grid[0], SPEC_NT, a_x, e->spec_smem[0]));
     if (e->spec_col) {
         CK(go(e->spec_yzy, e->spec_grid[3], SPEC_YZY_NT, a_s, e->spec_smem[3]));
@@ -883,6 +887,7 @@ cmsl_status spec_launch(Engine *e, cudaStream_t st, const Dev &d, const Fields<f
         CK(go(e->spec_y, e->spec_grid[1], SPEC_NT, a_s, e->spec_smem[1]));
     }
     CK(go(e->spec_x[1], e->spec_grid[0], SPEC_NT, a_x, e->spec_smem[0]));
+    if (e->spec_pin) CK(go((void *)k_spec_shift, e->spec_pin, SPEC_NT, a_x, 0));
     return CMSL_OK;
 }
 
@@ -1292,6 +1297,7 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
     int spec_mmax = 1;
     {
         bool want = false, forced = false, ok = e->precision != CMSL_FP64, anydep = false, ok_auto = true;
+        bool dirichlet = true;
         for (int i = 0; i < n; ++i) {
             const cmsl_film_desc &d = descs[i];
             forced |= d.inner_solver == CMSL_INNER_DIRECT;
@@ -1303,11 +1309,12 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
             // several permittivities: the solve preconditions the refinement
             // (AUTO up to SPEC_PRECOND_KAPPA, any ratio when DIRECT is asked for)
             ok_auto &= kappa <= SPEC_PRECOND_KAPPA;
-            ok &= d.zbc == CMSL_DIRICHLET && d.nz >= 3 && spec_radix_ok(d.nx) && spec_radix_ok(d.ny);
-            spec_mmax = std::max(spec_mmax, d.nz - 2);
+            ok &= d.nz >= 3 && spec_radix_ok(d.nx) && spec_radix_ok(d.ny);
+            dirichlet &= d.zbc == CMSL_DIRICHLET;
+            spec_mmax = std::max(spec_mmax, d.zbc == CMSL_DIRICHLET ? d.nz - 2 : d.nz);
         }
         ok &= anydep && spec_zthreads(spec_mmax) > 0;
-        if (forced && !ok)
+        if (forced && !(ok && dirichlet))
             return fail(CMSL_ERR_ARG, "inner_solver DIRECT needs FP32_REFINED films whose depolarisation solves have "
                                       "the Dirichlet z boundary and nx, ny of the form 2^a 3^b <= 4096");
         e->spectral = ok && want && (forced || ok_auto);
@@ -1556,7 +1563,7 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
         // per-film plans, tables and block ranges of the three passes
         const int zt = spec_zthreads(spec_mmax);
         std::vector<SpecFilm> sf((size_t)n);
-        std::vector<int> bxf, byf, bzf, bqf, bcf;
+        std::vector<int> bxf, byf, bzf, bqf, bcf, bnf;
         size_t smq = 0, smc = 0;
         int dev_o = 0, optin = 0;
         CK(cudaGetDevice(&dev_o));
@@ -1571,7 +1578,7 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
         bool cl_ok = clv && atoi(clv) != 0;
         for (int fi = 0; fi < n; ++fi)
             if (e->fh[fi].dep)
-                cl_ok = cl_ok && spec_cl_ok(spec_plan(e->fh[fi].nx), spec_plan(e->fh[fi].ny), e->fh[fi].nx,
+                cl_ok = cl_ok && e->fh[fi].zbc == CMSL_DIRICHLET && spec_cl_ok(spec_plan(e->fh[fi].nx), spec_plan(e->fh[fi].ny), e->fh[fi].nx,
                                             e->fh[fi].ny, (size_t)optin);
         e->spec_cl = cl_ok;
         long long ioff = 0;
@@ -1596,7 +1603,15 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
             P.bx0 = (int)bxf.size(); P.by0 = (int)byf.size(); P.bz0 = (int)bzf.size(); P.bq0 = (int)bqf.size();
             P.bc0 = (int)bcf.size();
             if (!h.dep) continue;                                    // no solve, no blocks
-            P.M = h.nz - 2;
+            P.neu = h.zbc != CMSL_DIRICHLET;
+            P.k0 = P.neu ? 0 : 1;
+            P.ref = fds[fi].ref_id;
+            P.M = h.nz - 2 * P.k0;
+            if (P.neu) {
+                P.bn0 = (int)bnf.size();
+                P.nbn = (int)((h.N + SPEC_PIN_CELLS - 1) / SPEC_PIN_CELLS);
+                bnf.insert(bnf.end(), (size_t)P.nbn, fi);
+            }
             P.Mp = (P.M + 1) / 2;
             P.ax = spec_plan(h.nx);
             P.ay = spec_plan(h.ny);
@@ -1668,7 +1683,11 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
                     const long long mode = e->spec_col ? (long long)kx * h.ny + ky : (long long)ky * h.nx + kx;
                     double c = 0.0;
                     for (int k = 0; k < P.M; ++k) {
-                        const double inv = 1.0 / (dg + c);
+                        // Neumann: the end rows halved; the zero mode's last pivot is
+                        // singular (its last plane stays 0)
+                        const bool end = P.neu && (k == 0 || k == P.M - 1);
+                        const bool sing = P.neu && k == P.M - 1 && kx == 0 && ky == 0;
+                        const double inv = sing ? 0.0 : 1.0 / ((end ? 0.5 * dg : dg) + c);
                         piv[(size_t)(P.ioff + k * modes + mode)] = (float)inv;
                         c = -inv;
                     }
@@ -1686,6 +1705,12 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
         TRY(upload(byf.data(), sizeof(int) * byf.size(), &p)); sp.by_film = (const int *)p;
         TRY(upload(bzf.data(), sizeof(int) * bzf.size(), &p)); sp.bz_film = (const int *)p;
         TRY(upload(bqf.data(), sizeof(int) * bqf.size(), &p)); sp.bq_film = (const int *)p;
+        e->spec_pin = (int)bnf.size();
+        sp.neu = !bnf.empty();
+        if (sp.neu) {
+            TRY(upload(bnf.data(), sizeof(int) * bnf.size(), &p)); sp.bn_film = (const int *)p;
+            TRY(e->alloc((void **)&sp.npart, sizeof(float2) * bnf.size()));
+        }
         if (bcf.empty()) bcf.push_back(0);
         TRY(upload(bcf.data(), sizeof(int) * bcf.size(), &p)); sp.bc_film = (const int *)p;
         TRY(upload(tw.data(), sizeof(float2) * tw.size(), &p)); sp.tw = (const float2 *)p;

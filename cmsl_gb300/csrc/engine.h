@@ -105,6 +105,7 @@ struct Engine {
     int spec_grid[5] = {0, 0, 0, 0, 0};   // blocks of the x, y, z passes, the column-pair pass, the cluster passes
     int spec_zt = 0;            // threads per block of the z solve
     size_t spec_smem[5] = {0, 0, 0, 0, 0};
+    int spec_pin = 0;           // blocks of k_spec_pin and k_spec_shift (films with the Neumann z boundary)
     bool spec_col = false;      // column layout: x, fused y-z-y, x (three launches per solve)
     bool spec_cl = false;       // column layout by cluster transforms: xy, z, yx (three launches per solve)
     bool persistent = false;

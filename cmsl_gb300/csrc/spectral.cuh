@@ -55,7 +55,11 @@ struct SpecFilm {
     SpecAxis ax, ay;
     long long off;              // first cell of the film
     long long coff;             // first spectrum value: [Mp][ny][nx], plane j = interior planes 2j, 2j+1
-    int nx, ny, nz, M, Mp;      // M = nz - 2 interior planes, Mp = ceil(M / 2) packed planes
+    int nx, ny, nz, M, Mp;      // M solved planes (Dirichlet: nz - 2 interior; Neumann: nz), Mp = ceil(M / 2) packed
+    int k0;                     // first solved plane (Dirichlet 1, Neumann 0)
+    int neu;                    // Neumann z boundary
+    int ref;                    // Neumann: the pinned cell
+    int bn0, nbn;               // Neumann: the film's blocks in the grids of k_spec_pin and k_spec_shift
     int twx, twy, lamx, lamy;   // offsets into the twiddle / eigenvalue tables
     float scale;                // h^2 / (eps nx ny)
     int bx0, by0, bz0;          // first block of the film in the x, y and z grids
@@ -78,6 +82,9 @@ struct SpecDev {
     // in the row layout), computed on the host in double: the z solves run
     // without divisions on their serial chain
     const float *piv;
+    const int *bn_film;         // film of every block of k_spec_pin and k_spec_shift (launches with Neumann films)
+    float2 *npart;              // their blocks' partial sums
+    int neu;                    // the launch has Neumann films: k_spec_shift ends the solve
 };
 
 __device__ __forceinline__ float2 c_add(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
@@ -408,9 +415,8 @@ __device__ __forceinline__ bool spec_run(const Dev &d, int f)
 // film's inner solve done (one "iteration").
 // Under deferred checks (Dev::defer, the solve node of a step) a step whose
 // films all end on this solve ends here.
-__device__ __forceinline__ void spec_finish(const Dev &d)
+__device__ __forceinline__ void spec_end(const Dev &d)
 {
-    if (!ticket_last(d.counter)) return;
     __shared__ int s_out;
     if (threadIdx.x == 0) {
         int out = 0;
@@ -429,6 +435,10 @@ __device__ __forceinline__ void spec_finish(const Dev &d)
     }
     __syncthreads();
     if (d.defer && d.step_end && !d.force && !s_out) step_end(d);
+}
+__device__ __forceinline__ void spec_finish(const Dev &d)
+{
+    if (ticket_last(d.counter)) spec_end(d);
 }
 
 // x transforms of rows (j, y) of the packed planes, j = 0 .. Mp-1.  IN_REAL:
@@ -461,7 +471,7 @@ __global__ void __launch_bounds__(SPEC_NT, 4) k_spec_x(Dev d, Fields<float> F, S
     extern __shared__ float2 sm2[];
     const int f = __ldg(sp.bx_film + blockIdx.x);
     if (!spec_run(d, f)) {
-        if (!IN_REAL) spec_finish(d);
+        if (!IN_REAL && !sp.neu) spec_finish(d);
         return;
     }
     const SpecFilm &P = sp.films[f];
@@ -472,7 +482,7 @@ __global__ void __launch_bounds__(SPEC_NT, 4) k_spec_x(Dev d, Fields<float> F, S
     float *xx = F.x + P.off;
     float2 *Cf = sp.C + P.coff;
     const SpecAxis &ax = P.ax;
-    const int M = P.M, Mp = P.Mp;
+    const int M = P.M, Mp = P.Mp, k0 = P.k0;
     // row pitch of the tiles: nx, or nx + 1 in the column layout, whose
     // transposed copies read a column of the tile (an odd pitch in 8-byte
     // words spreads its rows over the banks)
@@ -499,7 +509,7 @@ __global__ void __launch_bounds__(SPEC_NT, 4) k_spec_x(Dev d, Fields<float> F, S
     auto ld = [&](int sq, int e) -> float2 {
         if (!IN_REAL) return COL ? a[spec_pad(sq * pitch + e)] : Cf[(long long)(r0 + sq) * nx + e];
         const int rw = r0 + sq, j = rw / ny;
-        const long long o = (long long)(2 * j + 1) * plane + (long long)(rw - j * ny) * nx + e;
+        const long long o = (long long)(2 * j + k0) * plane + (long long)(rw - j * ny) * nx + e;
         return make_float2(rr[o], 2 * j + 1 < M ? rr[o + plane] : 0.f);
     };
     // the tile that receives the transform in the column layout's store
@@ -517,7 +527,7 @@ __global__ void __launch_bounds__(SPEC_NT, 4) k_spec_x(Dev d, Fields<float> F, S
         }
         // the transform of conj(W) is conj(x_2j + i x_2j+1) (scale folded into the z solve)
         const int rw = r0 + sq, j = rw / ny;
-        const long long yx = (long long)(rw - j * ny) * nx + e, o = (long long)(2 * j + 1) * plane + yx;
+        const long long yx = (long long)(rw - j * ny) * nx + e, o = (long long)(2 * j + k0) * plane + yx;
         if (cm != 0.f) {
             xx[o] = cw * v.x + cm * xx[o];
             if (2 * j + 1 < M) xx[o + plane] = cw * -v.y + cm * xx[o + plane];
@@ -525,8 +535,10 @@ __global__ void __launch_bounds__(SPEC_NT, 4) k_spec_x(Dev d, Fields<float> F, S
             xx[o] = cw * v.x;
             if (2 * j + 1 < M) xx[o + plane] = cw * -v.y;
         }
-        if (j == 0) xx[yx] = 0.f;                                        // first Dirichlet plane
-        if (j == Mp - 1) xx[(long long)(M + 1) * plane + yx] = 0.f;      // last one
+        if (k0) {
+            if (j == 0) xx[yx] = 0.f;                                    // first Dirichlet plane
+            if (j == Mp - 1) xx[(long long)(M + 1) * plane + yx] = 0.f;  // last one
+        }
     };
     __syncthreads();                                                     // twiddles
     fft_any<false, MIXED>(a, b, nr, ax, 1, pitch, tw, ld, st);
@@ -539,7 +551,7 @@ __global__ void __launch_bounds__(SPEC_NT, 4) k_spec_x(Dev d, Fields<float> F, S
             Cf[col_at(sq, e)] = res[spec_pad(sq * pitch + e)];
         }
     }
-    if (!IN_REAL) spec_finish(d);
+    if (!IN_REAL && !sp.neu) spec_finish(d);
 }
 
 // y transforms of column groups of one packed plane, in place on the
@@ -639,10 +651,11 @@ static __global__ void k_spec_z(Dev d, SpecDev sp)
         cp8(s + 1, Cb + j * modes);
     }
     cp_commit();
-    const float s = 0.5f * P.scale;
+    const float s0 = 0.5f * P.scale, s_end = P.neu ? 0.5f * s0 : s0;
     cp_wait<0>();
     float2 d_prev = make_float2(0.f, 0.f);
     auto sweep = [&](int k, float2 rk) {             // forward elimination (sub/super-diagonal -1)
+        const float s = k == 0 || k == M - 1 ? s_end : s0;       // Neumann: the end rows halved (SpecDev::piv)
         const float inv = pvs[(size_t)k * T];
         d_prev = make_float2((rk.x * s + d_prev.x) * inv, (rk.y * s + d_prev.y) * inv);
         return d_prev;
@@ -736,7 +749,7 @@ template <bool MIXED> __global__ void __launch_bounds__(SPEC_YZY_NT, 1) k_spec_y
     __syncthreads();
     // z solve, one thread per mode pair (as k_spec_z)
     const int npair = ncol == 2 ? ny : ny / 2 + 1;
-    const float s = 0.5f * P.scale;
+    const float s0 = 0.5f * P.scale, s_end = P.neu ? 0.5f * s0 : s0;
     for (int ky = threadIdx.x; ky < npair; ky += blockDim.x) {
         const int ky2 = ky == 0 ? 0 : ny - ky;
         const bool self = ncol == 1 && ky == ky2;
@@ -745,6 +758,7 @@ template <bool MIXED> __global__ void __launch_bounds__(SPEC_YZY_NT, 1) k_spec_y
         auto slot_b = [&](int j) { return &R[spec_pad((j * ncol + ncol - 1) * ny + ky2)]; };
         float2 d_prev = make_float2(0.f, 0.f);
         auto sweep = [&](int k, float2 rk) {     // forward elimination (sub/super-diagonal -1)
+            const float s = k == 0 || k == M - 1 ? s_end : s0;   // Neumann: the end rows halved (SpecDev::piv)
             const float inv = pv[k * ny];
             d_prev = make_float2((rk.x * s + d_prev.x) * inv, (rk.y * s + d_prev.y) * inv);
             return d_prev;
@@ -792,6 +806,98 @@ template <bool MIXED> __global__ void __launch_bounds__(SPEC_YZY_NT, 1) k_spec_y
     auto ld = [&](int sq, int e) { return R[spec_pad(sq * ny + e)]; };
     auto st = [&](int sq, int e, float2 v) { gcol(sq)[e] = v; };
     fft_any<false, MIXED>(R, R == A ? B : A, nseq, ay, 1, ny, tw, ld, st);
+}
+
+// ------------------------------------------------- Neumann z boundary
+// The mirrored end rows (depol_varEPS.cu:86-99) make every plane an unknown:
+// the tridiagonal systems run over all nz planes with end rows
+// (lam + 2) X_0 - 2 X_1 = s R_0, halved to keep them symmetric.  Without the
+// pinned cell the operator L is singular: constants c are in its kernel, and
+// L y = r' needs sum w r' = 0 with w = 1/2 on the end planes and 1 inside (the
+// zero mode's pivots end in a 0, which sets its last plane to 0).  The pinned
+// system (row ref: dx_ref = r_ref, the other rows L) is then solved by giving
+// r the value at the pinned cell that makes it compatible (k_spec_pin) --
+// that row of L is not among the system's rows -- and adding to the solution
+// the constant that puts r_ref there (k_spec_shift).  The persistent and
+// two-kernel PCG it stands in for took 380 to 1300 iterations a step (the pin
+// makes the operator ill-conditioned): 96x64x12 12.3 ms a step before.
+// Both kernels: a film's blocks share its cells; the film's last block (its
+// ticket from 4 on in Dev::counter) does the film's scalar part.
+constexpr int SPEC_PIN_CELLS = 8192;                            // cells of a block
+
+static __global__ void __launch_bounds__(SPEC_NT) k_spec_pin(Dev d, Fields<float> F, SpecDev sp)
+{
+    __shared__ double sRed[SPEC_NT / 32][1];
+    const int f = sp.bn_film[blockIdx.x];
+    if (!spec_run(d, f)) return;
+    const SpecFilm &P = sp.films[f];
+    const long long plane = (long long)P.nx * P.ny, n = plane * P.nz;
+    float *rr = F.r + P.off;
+    const int lb = (int)blockIdx.x - P.bn0;
+    const long long i1 = min(n, (long long)(lb + 1) * SPEC_PIN_CELLS);
+    df a{0.f, 0.f};
+    for (long long i = (long long)lb * SPEC_PIN_CELLS + threadIdx.x; i < i1; i += SPEC_NT) {
+        if (i == P.ref) continue;
+        a = df_add_f(a, i < plane || i >= n - plane ? 0.5f * rr[i] : rr[i]);
+    }
+    double v[1] = {(double)a.h + (double)a.l}, tot[1];
+    block_sum<1, double>(v, sRed, tot);
+    if (threadIdx.x == 0) {
+        const float h = (float)tot[0];
+        __stcg(sp.npart + blockIdx.x, make_float2(h, (float)(tot[0] - (double)h)));
+    }
+    __shared__ bool s_last;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        s_last = atomicAdd(d.counter + 4 + f, 1u) + 1u == (unsigned int)P.nbn;
+        if (s_last) d.counter[4 + f] = 0u;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    v[0] = 0.0;
+    for (int b = threadIdx.x; b < P.nbn; b += SPEC_NT) {
+        const float2 q = __ldcg(sp.npart + P.bn0 + b);
+        v[0] += (double)q.x + (double)q.y;
+    }
+    block_sum<1, double>(v, sRed, tot);
+    if (threadIdx.x == 0) {
+        SolveDev *S = d.solve + f;
+        S->pin_r = rr[P.ref];
+        S->pin_x = F.x[P.off + P.ref];
+        const bool end = P.ref < plane || P.ref >= n - plane;
+        rr[P.ref] = (float)(end ? -2.0 * tot[0] : -tot[0]);
+    }
+}
+
+// The constant: the increment at the pinned cell is w r_ref + m dx_ref as
+// elsewhere.  Every block reads the solution there; the last one of the grid
+// writes it.
+static __global__ void __launch_bounds__(SPEC_NT) k_spec_shift(Dev d, Fields<float> F, SpecDev sp)
+{
+    const int f = sp.bn_film[blockIdx.x];
+    if (spec_run(d, f)) {
+        const SpecFilm &P = sp.films[f];
+        const SolveDev *S = d.solve + f;
+        const long long n = (long long)P.nx * P.ny * P.nz;
+        float *xx = F.x + P.off;
+        const float want = d.force ? 0.f : S->cheb_w * S->pin_r + S->cheb_m * S->pin_x;
+        const float c = want - xx[P.ref];
+        const int lb = (int)blockIdx.x - P.bn0;
+        const long long i1 = min(n, (long long)(lb + 1) * SPEC_PIN_CELLS);
+        for (long long i = (long long)lb * SPEC_PIN_CELLS + threadIdx.x; i < i1; i += SPEC_NT)
+            if (i != P.ref) xx[i] += c;
+    }
+    if (!ticket_last(d.counter)) return;
+    if (threadIdx.x == 0)
+        for (int q = 0; q < d.n_films; ++q) {
+            const SpecFilm &P = sp.films[q];
+            const SolveDev *S = d.solve + q;
+            if (P.neu && spec_run(d, q)) F.x[P.off + P.ref] = d.force ? 0.f : S->cheb_w * S->pin_r + S->cheb_m * S->pin_x;
+        }
+    __syncthreads();
+    spec_end(d);
 }
 
 // ------------------------------------------------- cluster transforms
