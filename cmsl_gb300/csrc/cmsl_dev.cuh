@@ -44,6 +44,7 @@ template <int TYc> struct TileShape {
 };
 constexpr int TILE_YS[3] = {4, 8, 16};
 constexpr int P64_WORDS = 32;       // FP64 PCG: all-reduce words of a film (two sets, 128 bytes apart)
+constexpr int XSUM_W = 12;          // words of one accumulator of the FP32 passes' sums
 constexpr int NPART = 8;            // doubles of partial sums per item
 
 constexpr uint32_t GID_MASK = 0x00ffffffu;
@@ -120,8 +121,6 @@ struct SolveDev {               // per film, lives in device memory
     double cheb_rho;            // Chebyshev recurrence of the preconditioned refinement (rho_k)
     float cheb_w, cheb_m;       // the next direct solve's increment: dx <- w M^-1 r + m dx
     float pin_r, pin_x;         // direct solve of a Neumann film: r and the previous increment at the pinned cell
-    int row_pend;               // Dev::row_off: the sweep row (+1; 0 none) whose item partials the
-                                // TDGL step left for the next residual pass to total and write
     int pending;                // the step ended on its direct solve: the potential is phi_cur (the
                                 // warm start) + dx, its check r <- r - A dx still to come (next TDGL)
 };
@@ -169,23 +168,19 @@ struct FilmMaps {            // CUtensorMap carries its own alignment
     CUtensorMap dinv;           // 3D float (body)
 };
 
+// (A Dev above 256 bytes measured 1-2 us more per graph step.)
 struct Dev {
     const FilmDev *films;
     const int4 *items;
     int n_films, n_items;
     const int4 *sitems;         // items of the FP32 stencil passes (tile height of the autotuner's choice)
     int n_sitems;
-    int row_off;                // single films with deferred checks: block 0 of the step's first
-                                // residual pass totals and writes the TDGL step's sweep row
-                                // (SolveDev::row_pend) while the other blocks run their items.
-                                // (Kept in the padding after n_sitems: a Dev above 256 bytes
-                                // measured 1-2 us more per graph step.)
     const uint32_t *code;
     long long ncells;           // cells of all films (stride of the FP32 P pairs)
     double *phi[5];
-    double *partial;            // [n_items * NPART]
-    double *rpartial;           // [n_items * NPART] the FP32 residual passes' partial sums (apart from
-                                // the TDGL's, which the step's first residual pass may still total)
+    double *partial;            // [n_items * NPART] (FP64 passes and the two-kernel PCG)
+    unsigned long long *xsum;   // [n_films][2][8][XSUM_W] accumulators of the FP32 passes' sums (TDGL, residual),
+                                // zero between passes
     unsigned int *counter;      // [4 + n_films] the grid's ticket counter (reset by the last block);
                                 // from 4 on the per-film ones of the FP32 stencil passes (batches)
     SolveDev *solve;            // [n_films]

@@ -1482,8 +1482,8 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
     e->sitems_cap = std::max(count_items(e, ZCHUNK_MIN, TILE_YS[0]), count_items(e, 0, TILE_YS[0]));
     TRY(e->alloc((void **)&e->d_items, sizeof(int4) * e->items_cap));
     TRY(e->alloc((void **)&e->d_sitems, sizeof(int4) * e->sitems_cap));
-    e->part_cap = std::max(e->items_cap, e->sitems_cap);
-    TRY(e->alloc((void **)&e->d_partial, sizeof(double) * NPART * 2 * e->part_cap));
+    TRY(e->alloc((void **)&e->d_partial, sizeof(double) * NPART * e->items_cap));
+    if (e->precision != CMSL_FP64) TRY(e->alloc((void **)&e->d_xsum, sizeof(unsigned long long) * 16 * XSUM_W * n));
     {
         // tile height of the FP32 stencil passes: CMSL_TILE_Y (4, 8 or 16)
         // fixes it; else a tuned handle of the same shape class, else TY

@@ -243,14 +243,80 @@ __device__ __forceinline__ void film_total(const Dev &d, const FilmDev *f, doubl
     block_sum<NV, double>(v, sm, out);
 }
 
-// FP32 passes: the partial sums of an item are double-float pairs (float2
-// in the item's double slots) formed and added with FP32 instructions only,
-// so that neither the blocks' epilogues nor the last block's film totals
-// queue on the FP64 pipe.  The summation order is fixed (deterministic).
-template <int NV>
-__device__ __forceinline__ void block_partial32(const Dev &d, float (&v)[NV], double (*sm)[NV], double *part = nullptr)
+// FP32 passes: sums over a film's blocks as exact integers.  A block forms its
+// sum of each value in double-float, and adds both halves to the film's
+// accumulator of the value with 64-bit integer atomics: a float is a 24-bit
+// integer times a power of two, which falls on at most two of the
+// accumulator's nine 32-bit digits (units of 2^-149, digits kept in signed
+// 64-bit words that take 2^31 additions without carries).  The sum of the
+// blocks' pairs is exact, so it does not depend on their order or on the
+// tiling, and the last block reads a few words per value instead of every
+// item's pair: the total of eight values over 1024 items took it 8.6 k cycles
+// (loads of the pairs, double-float trees), now 1.5 k.
+// Words of a value: 9 digits, a count of non-finite contributions, 2 unused.
+__device__ __forceinline__ unsigned long long *xsum_words(const Dev &d, int fi, int kind)
 {
-    static_assert(NV <= 32, "one lane per value");
+    return d.xsum + (size_t)(fi * 2 + kind) * (8 * XSUM_W);
+}
+__device__ __forceinline__ void xsum_add(unsigned long long *w, float v)
+{
+    const unsigned int b = __float_as_uint(v), e = (b >> 23) & 255u;
+    if (e == 255u) {
+        atomicAdd(w + 9, 1ull);
+        return;
+    }
+    const unsigned int m = (b & 0x7fffffu) | (e ? 0x800000u : 0u);
+    if (!m) return;
+    const unsigned int sh = (e ? e : 1u) - 1u;
+    const unsigned long long u = (unsigned long long)m << (sh & 31u);
+    const unsigned long long lo = u & 0xffffffffull, hi = u >> 32;
+    const bool neg = (b >> 31) != 0u;
+    if (lo) atomicAdd(w + (sh >> 5), neg ? 0ull - lo : lo);
+    if (hi) atomicAdd(w + (sh >> 5) + 1, neg ? 0ull - hi : hi);
+}
+// The value of an accumulator's digits w (in shared memory, overwritten),
+// rounded once (the bits past the leading 64 cut).  Loops kept rolled: the
+// passes' kernels have no registers to spare.
+__device__ __forceinline__ double xsum_value(long long *w)
+{
+    #pragma unroll 1
+    for (int i = 0; i < 8; ++i) {
+        w[i + 1] += w[i] >> 32;
+        w[i] &= 0xffffffffll;
+    }
+    const bool neg = w[8] < 0;
+    if (neg) {                                      // negate: digits complemented, the carry through the zeros
+        long long carry = 1;
+        #pragma unroll 1
+        for (int i = 0; i < 8; ++i) {
+            const long long t = (w[i] ^ 0xffffffffll) + carry;
+            w[i] = t & 0xffffffffll;
+            carry = t >> 32;
+        }
+        w[8] = ~w[8] + carry;
+    }
+    if (w[9] != 0) return __longlong_as_double(0x7ff8000000000000ll);
+    int top = 8;
+    #pragma unroll 1
+    while (top > 0 && w[top] == 0) --top;
+    const unsigned long long m = (unsigned long long)w[top];     // the leading digit and the two below it
+    if (m == 0ull) return 0.0;
+    const unsigned long long n = ((unsigned long long)(top > 0 ? w[top - 1] : 0) << 32) |
+                                 (unsigned long long)(top > 1 ? w[top - 2] : 0);
+    const int lz = __clzll((long long)m);
+    const unsigned long long t = lz ? (m << lz) | (n >> (64 - lz)) : m;
+    const double v = __ull2double_rn(t);            // value = t 2^(32 top - lz - 149)
+    const double r = __hiloint2double(__double2hiint(v) + ((32 * top - lz - 149) << 20), __double2loint(v));
+    return neg ? -r : r;
+}
+
+// Adds the block's sums of NV values to film fi's accumulators (kind 0 the
+// TDGL step's, 1 the residual passes'): FP32 within a warp, double-float over
+// the warps.
+template <int NV>
+__device__ __forceinline__ void block_total32(const Dev &d, int fi, int kind, float (&v)[NV], double (*sm)[NV])
+{
+    static_assert(NV <= 8, "accumulators of a film");
     float *ws = (float *)&sm[0][0];               // [warps][NV] warp sums
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     #pragma unroll
@@ -259,71 +325,29 @@ __device__ __forceinline__ void block_partial32(const Dev &d, float (&v)[NV], do
         if (lane == 0) ws[w * NV + i] = s;
     }
     __syncthreads();
-    if (threadIdx.x < NV) {
+    if (threadIdx.x < 2 * NV) {                   // lane i the hi half of value i, lane NV + i the lo half
+        const int i = threadIdx.x < NV ? threadIdx.x : threadIdx.x - NV;
         const int nw = (int)(blockDim.x >> 5);
         df s{0.f, 0.f};
-        for (int q = 0; q < nw; ++q) s = df_add_f(s, ws[q * NV + threadIdx.x]);
-        *(float2 *)((part ? part : d.partial) + (long long)blockIdx.x * NPART + threadIdx.x) = make_float2(s.h, s.l);
+        for (int q = 0; q < nw; ++q) s = df_add_f(s, ws[q * NV + i]);
+        xsum_add(xsum_words(d, fi, kind) + i * XSUM_W, threadIdx.x < NV ? s.h : s.l);
     }
     __syncthreads();
 }
 
-// In the last block: film f's totals of the block_partial32 pairs of its
-// stencil items (Dev::sitems; item order: thread-strided U items a round,
-// warp tree, then warps in order), valid in thread 0.  The last block runs
-// alone at the end of its grid, so the sum is laid out for latency: every
-// load of a round is issued before its sums, and the values' warp trees
-// interleave.  OFF: the first slot; part: the partials (default the TDGL's).
-template <int NV, int OFF = 0>
-__device__ __forceinline__ void film_total32(const Dev &d, const FilmDev *f, double (*sm)[NV],
-                                             double (&out)[NV], const double *part = nullptr)
+// In the last block: film fi's totals of the NV values, valid in thread 0.
+template <int NV>
+__device__ __forceinline__ void film_total32(const Dev &d, int fi, int kind, double (&out)[NV])
 {
-    static_assert(OFF + NV <= NPART, "slots of an item");
-    const double *pp = part ? part : d.partial;
-    static_assert(NV <= 32 && sizeof(float2) == sizeof(double), "one lane and one slot per value");
+    __shared__ long long s_w[NV * XSUM_W];
     __shared__ double s_tot[NV];
-    float2 *ws = (float2 *)&sm[0][0];             // [warps][NV] warp totals
-    df v[NV];
-    #pragma unroll
-    for (int i = 0; i < NV; ++i) v[i] = df{0.f, 0.f};
-    const int b1 = f->sitem_end, stride = (int)blockDim.x;
-    auto ld = [&](int it, int i) { return __ldcg((const float2 *)(pp + (long long)it * NPART + OFF + i)); };
-    // U items a round, all their loads issued before the sums (about 16
-    // values in flight per thread: one round for a 1536-item film's single
-    // value instead of six)
-    constexpr int U = 16 / NV > 8 ? 8 : (16 / NV < 2 ? 2 : 16 / NV);
-    for (int it = f->sitem_begin + (int)threadIdx.x; it < b1; it += U * stride) {
-        float2 p[U][NV];
-        #pragma unroll
-        for (int u = 0; u < U; ++u)
-            #pragma unroll
-            for (int i = 0; i < NV; ++i)
-                p[u][i] = it + u * stride < b1 ? ld(it + u * stride, i) : make_float2(0.f, 0.f);
-        #pragma unroll
-        for (int u = 0; u < U; ++u)
-            #pragma unroll
-            for (int i = 0; i < NV; ++i) v[i] = df_add_acc(v[i], df{p[u][i].x, p[u][i].y});
-    }
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    #pragma unroll
-    for (int i = 0; i < NV; ++i) {
-        #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const df u{__shfl_down_sync(0xffffffffu, v[i].h, o), __shfl_down_sync(0xffffffffu, v[i].l, o)};
-            v[i] = df_add_acc(v[i], u);
-        }
-        if (lane == 0) ws[w * NV + i] = make_float2(v[i].h, v[i].l);
+    if (threadIdx.x < NV * XSUM_W) {                // every word in one round trip; cleared for the next pass
+        unsigned long long *w = xsum_words(d, fi, kind) + threadIdx.x;
+        s_w[threadIdx.x] = (long long)__ldcg(w);
+        __stcg(w, 0ull);
     }
     __syncthreads();
-    if (threadIdx.x < NV) {
-        const int nw = (int)(blockDim.x >> 5);
-        df s{0.f, 0.f};
-        for (int q = 0; q < nw; ++q) {
-            const float2 p = ws[q * NV + threadIdx.x];
-            s = df_add_acc(s, df{p.x, p.y});
-        }
-        s_tot[threadIdx.x] = (double)s.h + (double)s.l;
-    }
+    if (threadIdx.x < NV) s_tot[threadIdx.x] = xsum_value(s_w + threadIdx.x * XSUM_W);
     __syncthreads();
     if (threadIdx.x == 0) {
         #pragma unroll
@@ -399,7 +423,6 @@ __device__ __forceinline__ void op_z(const FilmDev *f, int k, V up, V dn, V &u, 
     else { u = dn; dd = dn; }
 }
 
-template <bool DF>
 __device__ __forceinline__ void tdgl_finish(const Dev &d, int rs, double (*sRed)[7], double (&sTot)[7]);
 
 // ---------------------------------------------------------- TDGL kernel
@@ -605,13 +628,12 @@ __global__ void __launch_bounds__(NT) k_tdgl(Dev d, Fields<T> F)
         }
     }
     if (!ticket_last(d.counter)) return;
-    tdgl_finish<false>(d, rs, sRed, sTot);
+    tdgl_finish(d, rs, sRed, sTot);
 }
 
 // Last block of a TDGL step: every film's sweep row from its items' partial
 // sums (evolve.cu:256-357 scaled as in :391-400), and the per-step reset of
 // the solver state.
-// DF: the partials are block_partial32 pairs (FP32 kernel).
 // Film fi's sweep row frow from the totals of its seven row sums (one thread).
 template <int NV>
 __device__ __forceinline__ void row_write(const Dev &d, int fi, int frow, const double (&sTot)[NV])
@@ -660,11 +682,11 @@ __device__ __forceinline__ void step_reopen(const Dev &d)
 // The FP32 TDGL step's end (finish32): film fi's sweep row and the reset of
 // its solver state; then the step's conditions.  Under kernel timing
 // (d.force) the totals are formed as a step forms them and nothing is written.
-__device__ __forceinline__ void tdgl_film32(const Dev &d, int rs, int fi, double (*sRed)[7], double (&sTot)[7])
+__device__ __forceinline__ void tdgl_film32(const Dev &d, int rs, int fi, double (&sTot)[7])
 {
     const int frow = d.rows[(long long)fi * d.wstride + rs];
     if (frow >= 0) {
-        film_total32<7>(d, d.films + fi, sRed, sTot);
+        film_total32<7>(d, fi, 0, sTot);
         if (threadIdx.x == 0 && !d.force) row_write(d, fi, frow, sTot);
     }
     if (threadIdx.x == 0 && !d.force) step_reset(d, fi);
@@ -679,15 +701,13 @@ __device__ __forceinline__ void tdgl_grid32(const Dev &d, int rs)
 
 // Under kernel timing (d.force) the totals are formed as a step forms them
 // and nothing is written.
-template <bool DF>
 __device__ __forceinline__ void tdgl_finish(const Dev &d, int rs, double (*sRed)[7], double (&sTot)[7])
 {
     for (int fi = 0; fi < d.n_films; ++fi) {
         const FilmDev *ff = d.films + fi;
         const int frow = d.rows[(long long)fi * d.wstride + rs];
         if (frow >= 0) {
-            if (DF) film_total32<7>(d, ff, sRed, sTot);
-            else film_total<7>(d, ff, sRed, sTot);
+            film_total<7>(d, ff, sRed, sTot);
             if (threadIdx.x == 0 && !d.force) row_write(d, fi, frow, sTot);
         }
         if (threadIdx.x == 0 && !d.force) step_reset(d, fi);
@@ -872,17 +892,17 @@ __device__ __forceinline__ void step_end(const Dev &d)
 // ||r|| <= refine_tol ||b||, rotates the buffers and sets the next inner
 // solve's target.
 // Film fi's part (finish32): its totals, the stop test and its next pass.
-__device__ __forceinline__ void refine_film(const Dev &d, int fi, double (*sRed)[3], double (&sTot)[3])
+__device__ __forceinline__ void refine_film(const Dev &d, int fi, double (&sTot)[3])
 {
     if (d.force) {              // kernel timing: the totals as a pass forms them; the state stays as it is
-        if (d.films[fi].dep_flag) film_total32<3>(d, d.films + fi, sRed, sTot, d.rpartial);
+        if (d.films[fi].dep_flag) film_total32<3>(d, fi, 1, sTot);
         return;
     }
     {
         const FilmDev *ff = d.films + fi;
         SolveDev *S = d.solve + fi;
         const bool was = ff->dep_flag != 0 && uniform_flag(&S->outer_active);
-        if (was) film_total32<3>(d, ff, sRed, sTot, d.rpartial);
+        if (was) film_total32<3>(d, fi, 1, sTot);
         if (threadIdx.x == 0 && was) {
             // an update pass (r <- r - A dx) leaves b.b as the last full pass formed it
             const bool was_upd = ff->upd_ok && S->upd && S->refine > 0;

@@ -248,7 +248,7 @@ template <int TYc, bool DEF = false> constexpr size_t t32_smem()
 }
 
 template <int NV>
-__device__ __forceinline__ void tdgl_def_film(const Dev &d, int rs, int fi, double (*sRed)[NV], double (&sTot)[NV]);
+__device__ __forceinline__ void tdgl_def_film(const Dev &d, int rs, int fi, double (&sTot)[NV]);
 __device__ __forceinline__ void tdgl_def_grid(const Dev &d, int rs);
 
 // TYc: the tile height (TX x TYc threads, one column each).
@@ -423,11 +423,11 @@ __global__ void __launch_bounds__(TileShape<TYc>::NTt, tdgl32_minb<TYc, DEF>()) 
     }
     cp_wait<0>();
 
-    if (row >= 0 || pend) block_partial32<NV>(d, acc, sRed);
+    if (row >= 0 || pend) block_total32<NV>(d, it.x, 0, acc, sRed);
     if constexpr (DEF)
-        finish32<FB>(d, [&](int fi) { tdgl_def_film<NV>(d, rs, fi, sRed, sTot); }, [&] { tdgl_def_grid(d, rs); });
+        finish32<FB>(d, [&](int fi) { tdgl_def_film<NV>(d, rs, fi, sTot); }, [&] { tdgl_def_grid(d, rs); });
     else
-        finish32<FB>(d, [&](int fi) { tdgl_film32(d, rs, fi, sRed, sTot); }, [&] { tdgl_grid32(d, rs); });
+        finish32<FB>(d, [&](int fi) { tdgl_film32(d, rs, fi, sTot); }, [&] { tdgl_grid32(d, rs); });
 }
 
 // The end of a TDGL step that may carry deferred checks (finish32): every
@@ -440,31 +440,21 @@ __global__ void __launch_bounds__(TileShape<TYc>::NTt, tdgl32_minb<TYc, DEF>()) 
 // whose checks passed stay pending (the repeated step checks them again, to
 // the same result), and the step loop runs this step again after that pass
 // has ended the previous one.
-// Film fi's part: its sweep row and its check's r.r (S->rr64).  Under
-// Dev::row_off the row is left to the step's first residual pass
-// (row_from_tdgl): only the check's r.r is totalled here, one value instead
-// of eight at the end of the grid.
+// Film fi's part: its sweep row and its check's r.r (S->rr64).
 template <int NV>
-__device__ __forceinline__ void tdgl_def_film(const Dev &d, int rs, int fi, double (*sRed)[NV], double (&sTot)[NV])
+__device__ __forceinline__ void tdgl_def_film(const Dev &d, int rs, int fi, double (&sTot)[NV])
 {
     static_assert(NV == 8, "seven row sums and the check's r.r");
     const FilmDev *ff = d.films + fi;
     SolveDev *S = d.solve + fi;
     const int frow = d.rows[(long long)fi * d.wstride + rs];
-    if (d.row_off) {
-        if (!ff->dep_flag || !(d.force || uniform_flag(&S->pending))) return;
-        double rr[1];
-        film_total32<1, NV - 1>(d, ff, (double (*)[1])sRed, rr);
-        if (threadIdx.x == 0 && !d.force) S->rr64 = rr[0];
-        return;
-    }
     if (d.force) {              // kernel timing: the totals as a step forms them; the state stays as it is
-        if (ff->dep_flag || frow >= 0) film_total32<NV>(d, ff, sRed, sTot);
+        if (ff->dep_flag || frow >= 0) film_total32<NV>(d, fi, 0, sTot);
         return;
     }
     const bool pend = ff->dep_flag != 0 && uniform_flag(&S->pending);
     if (frow < 0 && !pend) return;
-    film_total32<NV>(d, ff, sRed, sTot);
+    film_total32<NV>(d, fi, 0, sTot);
     if (threadIdx.x == 0) {
         if (frow >= 0) row_write(d, fi, frow, sTot);
         if (pend) S->rr64 = sTot[NV - 1];
@@ -502,10 +492,6 @@ __device__ __forceinline__ void tdgl_def_grid(const Dev &d, int rs)
                 S->pending = 0;
             }
             step_reset(d, fi);
-            if (d.row_off) {    // the step's first residual pass totals and writes the row
-                const int frow = d.rows[(long long)fi * d.wstride + rs];
-                S->row_pend = frow >= 0 ? frow + 1 : 0;
-            }
         }
         step_begin(d, rs);
     } else {
@@ -643,30 +629,6 @@ __device__ __forceinline__ void refine_cell(const RConst &rc, int k, bool ident,
     acc[2] = fmaf(rv, rv * wj, acc[2]);
 }
 
-__device__ __forceinline__ void refine_partials(const Dev &d, float (&acc)[3], double (*sRed)[3])
-{
-    block_partial32<3>(d, acc, sRed, d.rpartial);
-}
-
-// Dev::row_off (a single film with deferred checks): block 0 of the step's
-// first residual pass totals the sweep row from the TDGL step's item
-// partials (slots 0-6, which the residual passes leave alone) and writes it,
-// while the other blocks run their items; the TDGL step's last block formed
-// only the check's r.r.  Under kernel timing the total is formed and nothing
-// written.  Every thread of block 0.
-__device__ __forceinline__ void row_from_tdgl(const Dev &d, double (*sRow)[7])
-{
-    SolveDev *S = d.solve;
-    const int rp = d.force ? 1 : S->row_pend;
-    if (rp <= 0) return;
-    double t[7];
-    film_total32<7>(d, d.films, sRow, t);
-    if (threadIdx.x == 0 && !d.force) {
-        row_write(d, 0, rp - 1, t);
-        S->row_pend = 0;
-    }
-}
-
 // Stage layout (floats): x = phi (+ dx) as one (hi, lo) float2 plane, dx,
 // the (Pmx, Pmy) pair plane, Pmz (own), then the general-eps code and D^-1.
 // The update pass keeps the old r of the own cell in the Pmz slot.
@@ -691,10 +653,6 @@ __global__ void __launch_bounds__(TileShape<TYc>::NTt, TileShape<TYc>::MINB) k_r
     float *ring = (float *)smem_r32;
     __shared__ double sRed[NT / 32][3];
     __shared__ double sTot[3];
-    if (!FB && d.row_off && blockIdx.x == 0) {
-        __shared__ double sRow[NT / 32][7];
-        row_from_tdgl(d, sRow);
-    }
     const int4 it = d.sitems[blockIdx.x];
     const FilmDev *f = d.films + it.x;
     const SolveDev *S = d.solve + it.x;
@@ -807,8 +765,8 @@ __global__ void __launch_bounds__(TileShape<TYc>::NTt, TileShape<TYc>::MINB) k_r
         if (apply) nh[o] = make_float2(c.xc.h, c.xc.l);
     }
     cp_wait<0>();
-    refine_partials(d, acc, sRed);
-    finish32<FB>(d, [&](int fi) { refine_film(d, fi, sRed, sTot); }, [&] { refine_grid(d); });
+    if (run) block_total32<3>(d, it.x, 1, acc, sRed);
+    finish32<FB>(d, [&](int fi) { refine_film(d, fi, sTot); }, [&] { refine_grid(d); });
 }
 
 }  // namespace cmsl

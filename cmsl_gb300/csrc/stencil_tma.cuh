@@ -255,8 +255,8 @@ __global__ void __launch_bounds__(NT, 4) k_tdgl32t(Dev d, Fields<float> F)
         }
     }
 
-    if (row >= 0) block_partial32<7>(d, acc, sRed);
-    finish32<FB>(d, [&](int fi) { tdgl_film32(d, rs, fi, sRed, sTot); }, [&] { tdgl_grid32(d, rs); });
+    if (row >= 0) block_total32<7>(d, it.x, 0, acc, sRed);
+    finish32<FB>(d, [&](int fi) { tdgl_film32(d, rs, fi, sTot); }, [&] { tdgl_grid32(d, rs); });
 }
 
 // ------------------------------------------------- double-float residual
@@ -283,10 +283,6 @@ __global__ void __launch_bounds__(NT, 4) k_refine32t(Dev d, Fields<float> F)
     __shared__ TmaOp ops[RT_OPS];
     __shared__ double sRed[NT / 32][3];
     __shared__ double sTot[3];
-    if (!FB && d.row_off && blockIdx.x == 0) {
-        __shared__ double sRow[NT / 32][7];
-        row_from_tdgl(d, sRow);
-    }
     const int4 it = d.sitems[blockIdx.x];
     const FilmDev *f = d.films + it.x;
     const SolveDev *S = d.solve + it.x;
@@ -388,8 +384,8 @@ __global__ void __launch_bounds__(NT, 4) k_refine32t(Dev d, Fields<float> F)
         r[o] = rv;
         if (apply) nh[o] = make_float2(c.xc.h, c.xc.l);
     }
-    refine_partials(d, acc, sRed);
-    finish32<FB>(d, [&](int fi) { refine_film(d, fi, sRed, sTot); }, [&] { refine_grid(d); });
+    if (run) block_total32<3>(d, it.x, 1, acc, sRed);
+    finish32<FB>(d, [&](int fi) { refine_film(d, fi, sTot); }, [&] { refine_grid(d); });
 }
 
 
