@@ -44,7 +44,8 @@ template <int TYc> struct TileShape {
 };
 constexpr int TILE_YS[3] = {4, 8, 16};
 constexpr int P64_WORDS = 32;       // FP64 PCG: all-reduce words of a film (two sets, 128 bytes apart)
-constexpr int XSUM_W = 12;          // words of one accumulator of the FP32 passes' sums
+constexpr int XSUM_W = 12;          // words of one accumulator of the FP32 passes' sums,
+constexpr int XSUM_COPIES = 8;      // and copies of each
 constexpr int NPART = 8;            // doubles of partial sums per item
 
 constexpr uint32_t GID_MASK = 0x00ffffffu;
@@ -179,7 +180,7 @@ struct Dev {
     long long ncells;           // cells of all films (stride of the FP32 P pairs)
     double *phi[5];
     double *partial;            // [n_items * NPART] (FP64 passes and the two-kernel PCG)
-    unsigned long long *xsum;   // [n_films][2][8][XSUM_W] accumulators of the FP32 passes' sums (TDGL, residual),
+    unsigned long long *xsum;   // [n_films][2][XSUM_COPIES][8][XSUM_W] accumulators of the FP32 passes' sums (TDGL, residual),
                                 // zero between passes
     unsigned int *counter;      // [4 + n_films] the grid's ticket counter (reset by the last block);
                                 // from 4 on the per-film ones of the FP32 stencil passes (batches)

@@ -1483,7 +1483,7 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
     TRY(e->alloc((void **)&e->d_items, sizeof(int4) * e->items_cap));
     TRY(e->alloc((void **)&e->d_sitems, sizeof(int4) * e->sitems_cap));
     TRY(e->alloc((void **)&e->d_partial, sizeof(double) * NPART * e->items_cap));
-    if (e->precision != CMSL_FP64) TRY(e->alloc((void **)&e->d_xsum, sizeof(unsigned long long) * 16 * XSUM_W * n));
+    if (e->precision != CMSL_FP64) TRY(e->alloc((void **)&e->d_xsum, sizeof(unsigned long long) * 16 * XSUM_W * XSUM_COPIES * n));
     {
         // tile height of the FP32 stencil passes: CMSL_TILE_Y (4, 8 or 16)
         // fixes it; else a tuned handle of the same shape class, else TY

@@ -253,10 +253,13 @@ __device__ __forceinline__ void film_total(const Dev &d, const FilmDev *f, doubl
 // tiling, and the last block reads a few words per value instead of every
 // item's pair: the total of eight values over 1024 items took it 8.6 k cycles
 // (loads of the pairs, double-float trees), now 1.5 k.
-// Words of a value: 9 digits, a count of non-finite contributions, 2 unused.
+// Words of a value: 9 digits, a count of non-finite contributions, 2 unused;
+// XSUM_COPIES copies that the blocks take in turn (with one copy the atomics
+// of 1536 blocks queued: the 256x256x32 TDGL step at 32 x 4 tiles took 71
+// instead of 61 us).
 __device__ __forceinline__ unsigned long long *xsum_words(const Dev &d, int fi, int kind)
 {
-    return d.xsum + (size_t)(fi * 2 + kind) * (8 * XSUM_W);
+    return d.xsum + (size_t)(fi * 2 + kind) * (8 * XSUM_W * XSUM_COPIES);
 }
 __device__ __forceinline__ void xsum_add(unsigned long long *w, float v)
 {
@@ -330,7 +333,8 @@ __device__ __forceinline__ void block_total32(const Dev &d, int fi, int kind, fl
         const int nw = (int)(blockDim.x >> 5);
         df s{0.f, 0.f};
         for (int q = 0; q < nw; ++q) s = df_add_f(s, ws[q * NV + i]);
-        xsum_add(xsum_words(d, fi, kind) + i * XSUM_W, threadIdx.x < NV ? s.h : s.l);
+        xsum_add(xsum_words(d, fi, kind) + (blockIdx.x % XSUM_COPIES) * (8 * XSUM_W) + i * XSUM_W,
+                 threadIdx.x < NV ? s.h : s.l);
     }
     __syncthreads();
 }
@@ -342,9 +346,15 @@ __device__ __forceinline__ void film_total32(const Dev &d, int fi, int kind, dou
     __shared__ long long s_w[NV * XSUM_W];
     __shared__ double s_tot[NV];
     if (threadIdx.x < NV * XSUM_W) {                // every word in one round trip; cleared for the next pass
-        unsigned long long *w = xsum_words(d, fi, kind) + threadIdx.x;
-        s_w[threadIdx.x] = (long long)__ldcg(w);
-        __stcg(w, 0ull);
+        unsigned long long *w = xsum_words(d, fi, kind) + threadIdx.x, c[XSUM_COPIES], t = 0ull;
+        #pragma unroll
+        for (int q = 0; q < XSUM_COPIES; ++q) c[q] = __ldcg(w + q * (8 * XSUM_W));
+        #pragma unroll
+        for (int q = 0; q < XSUM_COPIES; ++q) {
+            t += c[q];
+            __stcg(w + q * (8 * XSUM_W), 0ull);
+        }
+        s_w[threadIdx.x] = (long long)t;
     }
     __syncthreads();
     if (threadIdx.x < NV) s_tot[threadIdx.x] = xsum_value(s_w + threadIdx.x * XSUM_W);
