@@ -93,6 +93,7 @@ struct FilmDev {
     double n_mat[3];            // voxels per material (sum of the reference's masks)
     Coef<double> coef[6];       // index mat*2 + iface
     Coef<float> coef32[6];
+    float coef_rot[6][12];      // the FP32 step's combined coefficients for orthonormal rotations (tdgl_cell32)
     double epsf[9];             // harmonic face eps for (mat_c, mat_nb), depol_varEPS.cu:10-15
     float epsf32[9];
     float cf_h[9], cf_l[9];     // epsf / h^2 as double-float pairs (FP32_REFINED residual)

@@ -329,6 +329,11 @@ void fill_film(FilmDev &fd, const cmsl_film_desc *dsc, int precision)
         for (int fl = 0; fl < 2; ++fl) {
             fill_coef<double>(fd.coef[mt * 2 + fl], dsc->mats[mt], fl, h, dsc->del_t);
             fill_coef<float>(fd.coef32[mt * 2 + fl], dsc->mats[mt], fl, h, dsc->del_t);
+            const Coef<double> &c = fd.coef[mt * 2 + fl];
+            const double r[9] = {6.0 * c.A + c.LdT * c.a02, c.A,          c.LdT,         c.LdT * (c.ag - c.a02),
+                                 c.LdT * (c.ags - c.a02), c.LdT * c.b4, c.LdT * c.b12, c.LdT * c.g6,
+                                 c.LdT * 5.0 * c.g6};
+            for (int q = 0; q < 12; ++q) fd.coef_rot[mt * 2 + fl][q] = q < 9 ? (float)r[q] : 0.f;
         }
     for (int a = 0; a < 3; ++a)
         for (int b = 0; b < 3; ++b) {
@@ -362,15 +367,32 @@ cmsl_status check_desc(const cmsl_film_desc *dsc, int idx, int n)
     return CMSL_OK;
 }
 
-// Rotations per grain: 9 values (FP64), or 9 values and 3 zeros (FP32: three
-// 16-byte loads per cell in the TDGL step).
+// Whether every rotation of the films is orthonormal (to rounding; the
+// reference's are products of three rotations, grain_io.cu:103-126).
+bool orthonormal_TR(const cmsl_film_desc *descs, int n)
+{
+    for (int i = 0; i < n; ++i)
+        for (int g = 0; g < descs[i].n_grains; ++g) {
+            const double *t = descs[i].TR + 9 * (size_t)g;
+            for (int a = 0; a < 3; ++a)
+                for (int b = a; b < 3; ++b) {
+                    const double v = t[3 * a] * t[3 * b] + t[3 * a + 1] * t[3 * b + 1] + t[3 * a + 2] * t[3 * b + 2];
+                    if (!(std::fabs(v - (a == b ? 1.0 : 0.0)) <= 1e-9)) return false;
+                }
+        }
+    return true;
+}
+
+// Rotations per grain: 9 values (FP64); FP32: the polar axis and a zero, or 9
+// values and 3 zeros where some rotation is not orthonormal.
 template <class T> cmsl_status upload_TR(Engine *e, const cmsl_film_desc *descs, int n)
 {
-    constexpr int stride = sizeof(T) == 4 ? TR32 : 9;
+    const bool axis = sizeof(T) == 4 && e->rot;
+    const int stride = sizeof(T) == 8 ? 9 : axis ? TR32_ROT : TR32_GEN, first = axis ? 6 : 0;
     std::vector<T> tr;
     for (int i = 0; i < n; ++i)
         for (int g = 0; g < descs[i].n_grains; ++g)
-            for (int q = 0; q < stride; ++q) tr.push_back(q < 9 ? (T)descs[i].TR[9 * g + q] : (T)0);
+            for (int q = first; q < first + stride; ++q) tr.push_back(q < 9 ? (T)descs[i].TR[9 * g + q] : (T)0);
     TRY(e->alloc(&e->d_TR, tr.size() * sizeof(T)));
     CK(cudaMemcpy(e->d_TR, tr.data(), tr.size() * sizeof(T), cudaMemcpyHostToDevice));
     return CMSL_OK;
@@ -1261,6 +1283,7 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
     e->precision = descs[0].precision;
     e->n_films = n;
     e->esz = e->precision == CMSL_FP64 ? 8 : 4;
+    e->rot = e->precision == CMSL_FP64 || orthonormal_TR(descs, n);
     const char *ng = getenv("CMSL_NO_GRAPH");
     e->use_graph = !(ng && atoi(ng) != 0);
     long long xy_tiles = 0;
@@ -1492,6 +1515,10 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
         const int ty_env = tyv ? atoi(tyv) : 0;
         e->tile_fixed = e->precision != CMSL_FP64 && (ty_env == 4 || ty_env == 8 || ty_env == 16);
         e->stile_ty = e->tile_fixed ? ty_env : TY;
+        if (!e->rot) {                  // general rotations: one tile shape
+            e->tile_fixed = true;
+            e->stile_ty = TY;
+        }
         std::lock_guard<std::mutex> lk(g_tuned_mu);
         const auto hit = g_tuned.find(shape_key(e));
         if (hit != g_tuned.end()) {
@@ -1782,6 +1809,7 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
         // the cp.async ring for all)
         const char *nt = getenv("CMSL_NO_TMA");
         e->tma = !(nt && atoi(nt) != 0);
+        e->tma = e->tma && e->rot;
         for (int fi = 0; fi < n; ++fi) e->tma = e->tma && e->fh[fi].nx % TX == 0 && e->fh[fi].ny % TY == 0;
         // the cp.async ring at every tile height, the tensor copies at TY
         // rows; batches take the kernels that finish each film in its own
@@ -1808,6 +1836,9 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
             e->tdgl_def[1] = (void *)k_tdgl32<T32_NS, 8, true>;
             e->tdgl_def[2] = (void *)k_tdgl32<T32_NS, 16, true>;
         }
+        if (!e->rot)                    // the rotations applied in full (tile height TY, no deferred checks)
+            for (void *&fn : e->tdgl_cp)
+                fn = fb ? (void *)k_tdgl32<T32_NS, TY, false, true, false> : (void *)k_tdgl32<T32_NS, TY, false, false, false>;
         e->refine_cp_smem[0] = uni ? r32_smem<true, 4>() : r32_smem<false, 4>();
         e->refine_cp_smem[1] = uni ? r32_smem<true, 8>() : r32_smem<false, 8>();
         e->refine_cp_smem[2] = uni ? r32_smem<true, 16>() : r32_smem<false, 16>();
@@ -1816,7 +1847,7 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
         e->tdgl_cp_smem[2] = t32_smem<16>();
         // deferred checks: some film's step can end on an exact direct solve
         const char *df = getenv("CMSL_DEFER");
-        e->defer = e->spectral && !e->persistent && !(df && atoi(df) == 0);
+        e->defer = e->spectral && !e->persistent && e->rot && !(df && atoi(df) == 0);
         bool any_def = false;
         for (int fi = 0; fi < n; ++fi) any_def |= fds[fi].defer_ok != 0;
         e->defer = e->defer && any_def;

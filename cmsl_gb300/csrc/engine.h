@@ -146,6 +146,7 @@ struct Engine {
         tdgl_nt = refine_nt = TX * stile_ty;
         graph_valid = false;
     }
+    bool rot = true;                    // every rotation orthonormal (the FP32 step needs the polar axes only)
     FilmMaps *d_maps = nullptr;
     int *d_err = nullptr;               // device error word
     CgBuf cg{};

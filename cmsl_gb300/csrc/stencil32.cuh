@@ -33,7 +33,9 @@
 
 namespace cmsl {
 
-constexpr int TR32 = 12;     // FP32 rotation per grain: 9 values + 3 pad (three 16-byte loads)
+// FP32 rotation per grain: films of orthonormal rotations keep the third row
+// and a pad (one 16-byte load), others 9 values and 3 pads (three).
+constexpr int TR32_ROT = 4, TR32_GEN = 12;
 
 // Warm start of a step's first refinement pass (own cell): 0 the previous
 // potential a, 1 linear 2a - q, 2 quadratic 3(a - q) + u, 3 cubic
@@ -138,11 +140,17 @@ __device__ __forceinline__ float minus_adx(const RConst &rc, int k, const RCell 
 // the extrapolated potential is written to the film's free buffer, which the
 // step's first residual pass then reads.
 
-// Coefficients of one (material, interface) class as three float4:
-// (relax, A, LdT, ag), (ags, b4, b12, g6), (a02, -, -, -).
-__device__ __forceinline__ void load_coef4(const FilmDev *f, float4 (*sC)[3])
+// Coefficients of one (material, interface) class as three float4: (relax, A,
+// LdT, ag), (ags, b4, b12, g6), (a02, -, -, -); ROT: FilmDev::coef_rot.
+template <bool ROT> __device__ __forceinline__ void load_coef4(const FilmDev *f, float4 (*sC)[3])
 {
     if (threadIdx.x < 6) {
+        if (ROT) {
+            const float *c = f->coef_rot[threadIdx.x];
+            #pragma unroll
+            for (int q = 0; q < 3; ++q) sC[threadIdx.x][q] = make_float4(c[4 * q], c[4 * q + 1], c[4 * q + 2], c[4 * q + 3]);
+            return;
+        }
         const Coef<float> &c = f->coef32[threadIdx.x];
         sC[threadIdx.x][0] = make_float4(c.relax, c.A, c.LdT, c.ag);
         sC[threadIdx.x][1] = make_float4(c.ags, c.b4, c.b12, c.g6);
@@ -198,14 +206,54 @@ __device__ __forceinline__ void load_tr32(const float4 *tr, float (&t)[9])
     t[4] = t1.x; t[5] = t1.y; t[6] = t1.z; t[7] = t1.w; t[8] = t2.x;
 }
 
-// The rotation loaded from the grain's entry tr.
-__device__ __forceinline__ void tdgl_cell32(const float4 *K, const float4 *tr, const float (&pc)[6],
+// The same for orthonormal rotations T (rows t1, t2, t3).  The transverse
+// restoring terms a02 act alike on both transverse directions, so
+//   T^T diag(a02, a02, d) T P = a02 P + (d - a02) (t3 . P) t3:
+// only the polar axis t3 is needed, one load of 16 bytes instead of three, and
+// the step is, with m = t3 . Pm, s = t3 . Ps and every coefficient times LdT,
+//   Pm' = Pm + (A sum - (6 A + LdT a02) Pm - m p(m, s) t3 - LdT E),
+//   p(m, s) = ag - a02 + m^2 (b4 + g6 (m^2 + 10 s^2)) + s^2 (b12 + 5 g6 s^2)
+// (kernels_evol.cu:162-229): 51 FP32 instructions for the two rotations there
+// and back, the Landau polynomials and the update, from about 97.  The
+// increment is formed apart: the rounding of a factor 1 - 6 A - LdT a02 would
+// recur every step (2.4e-6 instead of 7e-7 of error in P after 120 steps).
+// K: (6 A + LdT a02, A, LdT, ag'), (ags', b4', b12', g6'), (5 g6', -, -, -).
+__device__ __forceinline__ void tdgl_cell32r(const float4 *K, const float4 t, const float (&pc)[6],
+                                             const float (&sum)[6], float ex, float ey, float ez, float mEz,
+                                             float (&pn)[6], float &pMZl, float &pSZl)
+{
+    const float4 ka = K[0], kb = K[1];
+    const float g65 = K[2].x;
+    const float m = fmaf(t.z, pc[2], fmaf(t.y, pc[1], t.x * pc[0]));
+    const float s = fmaf(t.z, pc[5], fmaf(t.y, pc[4], t.x * pc[3]));
+    pMZl = m;
+    pSZl = s;
+    const float m2 = m * m, s2 = s * s;
+    const float um = fmaf(kb.w, fmaf(10.f, s2, m2), kb.y), us = fmaf(kb.w, fmaf(10.f, m2, s2), kb.y);
+    const float vm = fmaf(g65, s2, kb.z), vs = fmaf(g65, m2, kb.z);
+    const float qm = -m * fmaf(m2, um, fmaf(s2, vm, ka.w));
+    const float qs = -s * fmaf(s2, us, fmaf(m2, vs, kb.x));
+    const float tt[3] = {t.x, t.y, t.z}, e[3] = {ex, ey, mEz + ez};
+    #pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        pn[q] = pc[q] + fmaf(-ka.x, pc[q], fmaf(ka.y, sum[q], fmaf(qm, tt[q], -ka.z * e[q])));
+        pn[3 + q] = pc[3 + q] + fmaf(-ka.x, pc[3 + q], fmaf(ka.y, sum[3 + q], qs * tt[q]));
+    }
+}
+
+// One cell of grain entry gid of the film's rotations TR4.
+template <bool ROT>
+__device__ __forceinline__ void tdgl_cell32(const float4 *K, const float4 *TR4, int gid, const float (&pc)[6],
                                             const float (&sum)[6], float ex, float ey, float ez, float mEz,
                                             float (&pn)[6], float &pMZl, float &pSZl)
 {
-    float t[9];
-    load_tr32(tr, t);
-    tdgl_cell32t(K, t, pc, sum, ex, ey, ez, mEz, pn, pMZl, pSZl);
+    if (ROT) {
+        tdgl_cell32r(K, __ldg(TR4 + gid), pc, sum, ex, ey, ez, mEz, pn, pMZl, pSZl);
+    } else {
+        float t[9];
+        load_tr32(TR4 + 3LL * gid, t);
+        tdgl_cell32t(K, t, pc, sum, ex, ey, ez, mEz, pn, pMZl, pSZl);
+    }
 }
 
 // z neighbours of the potential for E (depol_varEPS.cu:246-273): zero beyond
@@ -269,7 +317,7 @@ template <int TYc, bool DEF> constexpr int tdgl32_minb()
     return DEF && TYc < 16 ? TileShape<TYc>::MINB * 3 / 4 : TileShape<TYc>::MINB;
 }
 
-template <int NS, int TYc = TY, bool DEF = false, bool FB = false>
+template <int NS, int TYc = TY, bool DEF = false, bool FB = false, bool ROT = true>
 __global__ void __launch_bounds__(TileShape<TYc>::NTt, tdgl32_minb<TYc, DEF>()) k_tdgl32(Dev d, Fields<float> F)
 {
     static_assert(NS >= 4, "the ring holds planes k-1, k, k+1 and at least one in flight");
@@ -284,7 +332,7 @@ __global__ void __launch_bounds__(TileShape<TYc>::NTt, tdgl32_minb<TYc, DEF>()) 
     const int4 it = d.sitems[blockIdx.x];
     const FilmDev *f = d.films + it.x;
     const int z0 = it.w & 0xffff, z1 = it.w >> 16;
-    load_coef4(f, sC);
+    load_coef4<ROT>(f, sC);
     const Geom g = make_geom<TYc>(f, it.y, it.z);
     const int cur = d.ctl->cur, rs = d.ctl->run_step;
     const float mEz = (float)(-d.wave[(long long)it.x * d.wstride + rs]);   // dfdPmz_app, kernels_evol.cu:210
@@ -304,7 +352,7 @@ __global__ void __launch_bounds__(TileShape<TYc>::NTt, tdgl32_minb<TYc, DEF>()) 
     float2 *xh = phi2_sel(d, phi_free(S)) + off;     // DEF: the checked potential x0 + dx
     const float *dxg = F.x + off, *rg = F.r + off;
     const uint32_t *code = d.code + off;
-    const float4 *TR4 = (const float4 *)(F.TR + (long long)TR32 * f->g_off);
+    const float4 *TR4 = (const float4 *)(F.TR + (long long)(ROT ? TR32_ROT : TR32_GEN) * f->g_off);
     const float2 *Po = pairs32(F, cur) + off;   // the three pairs of a set at j * fs
     float2 *Pn = pairs32(F, cur ^ 1) + off;
     const int zlo = max(z0 - 1, 0), zhi = min(z1, nz - 1);
@@ -410,8 +458,7 @@ __global__ void __launch_bounds__(TileShape<TYc>::NTt, tdgl32_minb<TYc, DEF>()) 
             ez *= inv_2hf;
         }
         float pn[6], pMZl, pSZl;
-        tdgl_cell32(sC[code_mat(c) * 2 + code_iface(c)], TR4 + 3LL * code_gid(c), pc, sum, ex, ey, ez, mEz, pn,
-                    pMZl, pSZl);
+        tdgl_cell32<ROT>(sC[code_mat(c) * 2 + code_iface(c)], TR4, code_gid(c), pc, sum, ex, ey, ez, mEz, pn, pMZl, pSZl);
         #pragma unroll
         for (int j = 0; j < 3; ++j) Pn[j * fs + o] = make_float2(pn[2 * j], pn[2 * j + 1]);
         if (row >= 0) row_acc(acc, code_mat(c), pn, pMZl, pSZl);
