@@ -82,30 +82,47 @@ double harm(double a, double b)   // depol_varEPS.cu:10-15
 
 namespace {
 
-// z chunk of the stencil items (xy_tiles: the column tiles of all films of
-// the handle together); CMSL_ZCHUNK overrides.
-int pick_zchunk(long long xy_tiles, int nz)
+// z chunk of the stencil items of a film of nz planes, for the column tiles of
+// all films of the handle together; CMSL_ZCHUNK overrides.
+// FP32: the chunk count with the least waves x (chunk + 6 planes): a block's
+// prologue (two halo planes, the first copies' latency) and its sums cost about
+// six planes, and a partial wave costs a whole one.  slots: resident blocks
+// (152 SMs x 3 for the TDGL step with checks, x 4 else).  At least 4 planes,
+// as the autotuner's candidates (256x256x32: 11 planes 145.4 us a step, 8
+// planes 147.2; 512x512x64: 32 planes 819, 64 planes 841; 128x128x16: 4 planes
+// 60.7, 8 planes 63.9; 64x64x16: 4 planes 53, 8 planes 61).
+// FP64: every SM's FP64 pipe serves all its blocks, so the least planes on the
+// most loaded SM (64x64x16: 2 planes on 128 blocks, the TDGL step 133 -> 42 us).
+int pick_zchunk(const Engine *e, int nz, int ty)
 {
     const char *env = getenv("CMSL_ZCHUNK");
     if (env && atoi(env) > 0) return std::min(nz, atoi(env));
-    // about 1.5 waves of the stencil passes (4 resident blocks on each of
-    // 152 SMs), chunks of at least 8 planes: the ring prologue and the two
-    // halo planes of a chunk cost more than the tail of a partial wave
-    const long long target = 6LL * 152;
-    const long long chunks = (target + xy_tiles - 1) / xy_tiles;
-    int zc = (int)std::max<long long>(1, (nz + chunks - 1) / chunks);
-    zc = std::max(zc, std::min(nz, 8));
-    return std::min(zc, nz);
+    const bool fp64 = e->precision == CMSL_FP64;
+    const long long tiles = e->xy_tiles[Engine::ty_index(ty)];
+    const long long slots = fp64 ? 152 : 152LL * (e->defer ? 3 : 4) * TY / ty;
+    const double lead = fp64 ? 0.5 : 6.0;
+    int best = nz;
+    double cost = 0.0;
+    for (int nc = 1; nc <= nz; ++nc) {
+        const int zc = (nz + nc - 1) / nc;
+        if (!fp64 && nc > 1 && zc < 4) break;
+        const double c = (double)((tiles * nc + slots - 1) / slots) * (zc + lead);
+        if (nc == 1 || c < cost) {
+            cost = c;
+            best = zc;
+        }
+    }
+    return best;
 }
 
 // Work items of every film for z chunk zc (0: pick_zchunk per film); how
 // many there are, or the items themselves with each film's item range.
 constexpr int ZCHUNK_MIN = 4;       // the finest chunk the autotuner tries
 
-int film_zchunk(const Engine *e, int fi, int zc)
+int film_zchunk(const Engine *e, int fi, int zc, int ty)
 {
     const int nz = e->fh[fi].nz;
-    return zc > 0 ? std::min(zc, nz) : pick_zchunk(e->xy_tiles, nz);
+    return zc > 0 ? std::min(zc, nz) : pick_zchunk(e, nz, ty);
 }
 
 // A column of nz planes in chunks of at most c planes: ceil(nz / c) chunks
@@ -119,7 +136,7 @@ size_t count_items(const Engine *e, int zc, int ty = TY)
     size_t n = 0;
     for (int fi = 0; fi < e->n_films; ++fi) {
         const FilmHost &h = e->fh[fi];
-        const int c = film_zchunk(e, fi, zc);
+        const int c = film_zchunk(e, fi, zc, ty);
         n += (size_t)((h.nx + TX - 1) / TX) * ((h.ny + ty - 1) / ty) * z_chunks(h.nz, c);
     }
     return n;
@@ -139,7 +156,7 @@ cmsl_status set_items(Engine *e, int zc)
         v.clear();
         for (int fi = 0; fi < e->n_films; ++fi) {
             const FilmHost &h = e->fh[fi];
-            const int nc = z_chunks(h.nz, film_zchunk(e, fi, zc));
+            const int nc = z_chunks(h.nz, film_zchunk(e, fi, zc, ty));
             FilmDev &fd = e->fdh[fi];
             (list ? fd.sitem_begin : fd.item_begin) = (int)v.size();
             for (int y0 = 0; y0 < h.ny; y0 += ty)
@@ -1286,7 +1303,6 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
     e->rot = e->precision == CMSL_FP64 || orthonormal_TR(descs, n);
     const char *ng = getenv("CMSL_NO_GRAPH");
     e->use_graph = !(ng && atoi(ng) != 0);
-    long long xy_tiles = 0;
     for (int i = 0; i < n; ++i) {
         const cmsl_film_desc &d = descs[i];
         FilmHost h;
@@ -1296,7 +1312,8 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
         e->ncells = h.off + h.N;
         e->fh.push_back(h);
         e->any_dep |= h.dep != 0;
-        xy_tiles += (long long)((d.nx + TX - 1) / TX) * ((d.ny + TY - 1) / TY);
+        for (int q = 0; q < 3; ++q)
+            e->xy_tiles[q] += (long long)((d.nx + TX - 1) / TX) * ((d.ny + TILE_YS[q] - 1) / TILE_YS[q]);
         e->max_iter_cap = std::max(e->max_iter_cap, d.max_iter);
         e->max_refine_cap = std::max(e->max_refine_cap, std::max(1, d.max_refine));
         e->inner_max_cap = std::max(e->inner_max_cap, std::max(1, d.inner_max_iter));
@@ -1408,7 +1425,6 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
         fd.g_off = g_off;
         g_off += h.ng;
     }
-    e->xy_tiles = xy_tiles;
 
     // persistent PCG partition: stencil bricks of PZ planes film by film;
     // each film gets a contiguous block range in proportion to its cells
@@ -1497,12 +1513,20 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
         const char *hd = getenv("CMSL_HOST_COPY");   // 1: host-side conversion and copies
         e->host_direct = pageable && host_tables && !(hd && atoi(hd) != 0);
     }
+    {
+        // deferred checks: some film's step can end on an exact direct solve
+        const char *df = getenv("CMSL_DEFER");
+        bool any_def = false;
+        for (int fi = 0; fi < n; ++fi) any_def |= fds[fi].defer_ok != 0;
+        e->defer = e->spectral && !e->persistent && e->rot && any_def && !(df && atoi(df) == 0);
+    }
     TRY(e->alloc((void **)&e->d_code, sizeof(uint32_t) * cells));
     TRY(build_film_codes(e, descs, fds));
     e->fdh = fds;
     TRY(e->alloc((void **)&e->d_films, sizeof(FilmDev) * n));
     e->items_cap = std::max(count_items(e, ZCHUNK_MIN), count_items(e, 0));
-    e->sitems_cap = std::max(count_items(e, ZCHUNK_MIN, TILE_YS[0]), count_items(e, 0, TILE_YS[0]));
+    e->sitems_cap = count_items(e, ZCHUNK_MIN, TILE_YS[0]);
+    for (int ty : TILE_YS) e->sitems_cap = std::max(e->sitems_cap, count_items(e, 0, ty));
     TRY(e->alloc((void **)&e->d_items, sizeof(int4) * e->items_cap));
     TRY(e->alloc((void **)&e->d_sitems, sizeof(int4) * e->sitems_cap));
     TRY(e->alloc((void **)&e->d_partial, sizeof(double) * NPART * e->items_cap));
@@ -1845,12 +1869,6 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
         e->tdgl_cp_smem[0] = t32_smem<4>();
         e->tdgl_cp_smem[1] = t32_smem<8>();
         e->tdgl_cp_smem[2] = t32_smem<16>();
-        // deferred checks: some film's step can end on an exact direct solve
-        const char *df = getenv("CMSL_DEFER");
-        e->defer = e->spectral && !e->persistent && e->rot && !(df && atoi(df) == 0);
-        bool any_def = false;
-        for (int fi = 0; fi < n; ++fi) any_def |= fds[fi].defer_ok != 0;
-        e->defer = e->defer && any_def;
         e->tdgl_def_smem[0] = t32_smem<4, true>();
         e->tdgl_def_smem[1] = t32_smem<8, true>();
         e->tdgl_def_smem[2] = t32_smem<16, true>();
@@ -1875,8 +1893,10 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
         }
         // CMSL_STAGING=<tdgl><residual> (digits 0 cp.async ring, 1 tensor
         // copies) fixes the staging of films with full tiles; the autotuner
-        // then keeps it
-        int st_t = STG_TMA, st_r = STG_TMA;
+        // then keeps it.  The ring until tuned: 256x256x32 147.2 us a step
+        // against 152.7 with the residual passes by tensor copies (first pass
+        // 30.9 / 35.1), 512x512x64 841 / 888, three permittivities 463 / 484
+        int st_t = STG_CP, st_r = STG_CP;
         const char *sg = getenv("CMSL_STAGING");
         e->staging_fixed = false;
         if (sg && strlen(sg) == 2 && sg[0] >= '0' && sg[0] < '0' + N_STG && sg[1] >= '0' && sg[1] < '0' + N_STG) {

@@ -58,7 +58,7 @@ struct Engine {
     std::vector<int4> sitems;           // items of the FP32 stencil passes (tile height stile_ty)
     size_t sitems_cap = 0;
     int stile_ty = TY;
-    long long xy_tiles = 0;             // column tiles of all films
+    long long xy_tiles[3] = {0, 0, 0};  // column tiles of all films, per tile height of TILE_YS
     int zchunk = 0;                     // z chunk of the items (0: per-film heuristic)
     // device buffers
     std::vector<void *> allocs;
@@ -112,7 +112,7 @@ struct Engine {
     // staging of the FP32 stencil passes: STG_CP the cp.async ring (any
     // film), STG_TMA tensor copies (every film's nx % 32 == 0, ny % 8 == 0).
     // The TDGL and the residual passes each take the staging the autotuner
-    // measured faster (STG_TMA until tuned)
+    // measured faster (the ring until tuned)
     // The cp.async ring has a kernel per tile height (TILE_YS: 4, 8, 16 rows
     // of 32 columns); the tensor copies run 8-row tiles only.
     bool tma = false;
