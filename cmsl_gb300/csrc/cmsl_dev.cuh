@@ -44,8 +44,7 @@ template <int TYc> struct TileShape {
 };
 constexpr int TILE_YS[3] = {4, 8, 16};
 constexpr int P64_WORDS = 32;       // FP64 PCG: all-reduce words of a film (two sets, 128 bytes apart)
-constexpr int XSUM_W = 12;          // words of one accumulator of the FP32 passes' sums,
-constexpr int XSUM_COPIES = 8;      // and copies of each
+constexpr int XSUM_W = 12;          // words of one accumulator of the FP32 passes' sums
 constexpr int NPART = 8;            // doubles of partial sums per item
 
 constexpr uint32_t GID_MASK = 0x00ffffffu;
@@ -88,9 +87,11 @@ struct FilmDev {
                                 // the half-width of M^-1 A's spectrum around 1 (0: exact solve)
     int upd_ok;                 // FP32_REFINED: the inner solve leaves r intact (direct solve), so a
                                 // later refinement pass may update r instead of recomputing it
+    int direct;                 // FP32_REFINED inner solve by the direct spectral solve
     int defer_ok;               // the check after a step's one direct solve may run inside the next
                                 // TDGL step (upd_ok, warm start at most quadratic)
     double n_mat[3];            // voxels per material (sum of the reference's masks)
+    double rowc[11];            // sweep row: factors of the sums, constants (evolve.cu:391-400)
     Coef<double> coef[6];       // index mat*2 + iface
     Coef<float> coef32[6];
     float coef_rot[6][12];      // the FP32 step's combined coefficients for orthonormal rotations (tdgl_cell32)
@@ -120,7 +121,7 @@ struct SolveDev {               // per film, lives in device memory
     int inner_max;              // inner iteration cap of the current pass
     int upd;                    // the next refinement pass updates r <- r - A dx (FP32) instead of
                                 // forming b - A phi in double-float
-    double cheb_rho;            // Chebyshev recurrence of the preconditioned refinement (rho_k)
+    float cheb_rho;             // Chebyshev recurrence of the preconditioned refinement (rho_k)
     float cheb_w, cheb_m;       // the next direct solve's increment: dx <- w M^-1 r + m dx
     float pin_r, pin_x;         // direct solve of a Neumann film: r and the previous increment at the pinned cell
     int pending;                // the step ended on its direct solve: the potential is phi_cur (the
@@ -181,7 +182,7 @@ struct Dev {
     long long ncells;           // cells of all films (stride of the FP32 P pairs)
     double *phi[5];
     double *partial;            // [n_items * NPART] (FP64 passes and the two-kernel PCG)
-    unsigned long long *xsum;   // [n_films][2][XSUM_COPIES][8][XSUM_W] accumulators of the FP32 passes' sums (TDGL, residual),
+    unsigned long long *xsum;   // [n_films][2][8][XSUM_W] accumulators of the FP32 passes' sums (TDGL, residual),
                                 // zero between passes
     unsigned int *counter;      // [4 + n_films] the grid's ticket counter (reset by the last block);
                                 // from 4 on the per-film ones of the FP32 stencil passes (batches)

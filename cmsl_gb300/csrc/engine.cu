@@ -1410,6 +1410,7 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
         // the FP32 update pass r <- r - A dx follows an exact (one-eps) direct solve only;
         // its check may run inside the next TDGL step when that step's warm start
         // leaves the third-oldest potential unread
+        fd.direct = e->spectral ? 1 : 0;
         fd.upd_ok = e->spectral && fd.uni_eps ? 1 : 0;
         fd.defer_ok = fd.upd_ok && fd.dep_flag && fd.warm <= 2 ? 1 : 0;
         fd.cheb_delta = 0.f;
@@ -1522,6 +1523,17 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
     }
     TRY(e->alloc((void **)&e->d_code, sizeof(uint32_t) * cells));
     TRY(build_film_codes(e, descs, fds));
+    for (FilmDev &fd : fds) {
+        const double N = (double)fd.nx * fd.ny * fd.nz;
+        for (int q = 0; q < 4; ++q) fd.rowc[q] = fd.inv_N;
+        static const int mat[3] = {1, 0, 2};                 // row order FE, AFE, DE
+        for (int q = 0; q < 3; ++q) {
+            const double nm = fd.n_mat[mat[q]];
+            fd.rowc[4 + 2 * q] = nm > 0.0 ? 1.0 / nm : 0.0;
+            fd.rowc[5 + 2 * q] = nm > 0.0 ? nm / N : 0.0;
+        }
+        fd.rowc[10] = 0.0;
+    }
     e->fdh = fds;
     TRY(e->alloc((void **)&e->d_films, sizeof(FilmDev) * n));
     e->items_cap = std::max(count_items(e, ZCHUNK_MIN), count_items(e, 0));
@@ -1530,7 +1542,7 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
     TRY(e->alloc((void **)&e->d_items, sizeof(int4) * e->items_cap));
     TRY(e->alloc((void **)&e->d_sitems, sizeof(int4) * e->sitems_cap));
     TRY(e->alloc((void **)&e->d_partial, sizeof(double) * NPART * e->items_cap));
-    if (e->precision != CMSL_FP64) TRY(e->alloc((void **)&e->d_xsum, sizeof(unsigned long long) * 16 * XSUM_W * XSUM_COPIES * n));
+    if (e->precision != CMSL_FP64) TRY(e->alloc((void **)&e->d_xsum, sizeof(unsigned long long) * 16 * XSUM_W * n));
     {
         // tile height of the FP32 stencil passes: CMSL_TILE_Y (4, 8 or 16)
         // fixes it; else a tuned handle of the same shape class, else TY

@@ -251,15 +251,13 @@ __device__ __forceinline__ void film_total(const Dev &d, const FilmDev *f, doubl
 // 64-bit words that take 2^31 additions without carries).  The sum of the
 // blocks' pairs is exact, so it does not depend on their order or on the
 // tiling, and the last block reads a few words per value instead of every
-// item's pair: the total of eight values over 1024 items took it 8.6 k cycles
-// (loads of the pairs, double-float trees), now 1.5 k.
-// Words of a value: 9 digits, a count of non-finite contributions, 2 unused;
-// XSUM_COPIES copies that the blocks take in turn (with one copy the atomics
-// of 1536 blocks queued: the 256x256x32 TDGL step at 32 x 4 tiles took 71
-// instead of 61 us).
+// item's pair (the total of eight values over 1024 items took it 8.6 k cycles:
+// loads of the pairs, double-float trees).
+// Words of a value: 9 digits, a count of non-finite contributions, 2 unused.
+// (Eight copies that the blocks take in turn measured no faster.)
 __device__ __forceinline__ unsigned long long *xsum_words(const Dev &d, int fi, int kind)
 {
-    return d.xsum + (size_t)(fi * 2 + kind) * (8 * XSUM_W * XSUM_COPIES);
+    return d.xsum + (size_t)(fi * 2 + kind) * (8 * XSUM_W);
 }
 __device__ __forceinline__ void xsum_add(unsigned long long *w, float v)
 {
@@ -277,42 +275,6 @@ __device__ __forceinline__ void xsum_add(unsigned long long *w, float v)
     if (lo) atomicAdd(w + (sh >> 5), neg ? 0ull - lo : lo);
     if (hi) atomicAdd(w + (sh >> 5) + 1, neg ? 0ull - hi : hi);
 }
-// The value of an accumulator's digits w (in shared memory, overwritten),
-// rounded once (the bits past the leading 64 cut).  Loops kept rolled: the
-// passes' kernels have no registers to spare.
-__device__ __forceinline__ double xsum_value(long long *w)
-{
-    #pragma unroll 1
-    for (int i = 0; i < 8; ++i) {
-        w[i + 1] += w[i] >> 32;
-        w[i] &= 0xffffffffll;
-    }
-    const bool neg = w[8] < 0;
-    if (neg) {                                      // negate: digits complemented, the carry through the zeros
-        long long carry = 1;
-        #pragma unroll 1
-        for (int i = 0; i < 8; ++i) {
-            const long long t = (w[i] ^ 0xffffffffll) + carry;
-            w[i] = t & 0xffffffffll;
-            carry = t >> 32;
-        }
-        w[8] = ~w[8] + carry;
-    }
-    if (w[9] != 0) return __longlong_as_double(0x7ff8000000000000ll);
-    int top = 8;
-    #pragma unroll 1
-    while (top > 0 && w[top] == 0) --top;
-    const unsigned long long m = (unsigned long long)w[top];     // the leading digit and the two below it
-    if (m == 0ull) return 0.0;
-    const unsigned long long n = ((unsigned long long)(top > 0 ? w[top - 1] : 0) << 32) |
-                                 (unsigned long long)(top > 1 ? w[top - 2] : 0);
-    const int lz = __clzll((long long)m);
-    const unsigned long long t = lz ? (m << lz) | (n >> (64 - lz)) : m;
-    const double v = __ull2double_rn(t);            // value = t 2^(32 top - lz - 149)
-    const double r = __hiloint2double(__double2hiint(v) + ((32 * top - lz - 149) << 20), __double2loint(v));
-    return neg ? -r : r;
-}
-
 // Adds the block's sums of NV values to film fi's accumulators (kind 0 the
 // TDGL step's, 1 the residual passes'): FP32 within a warp, double-float over
 // the warps.
@@ -333,38 +295,58 @@ __device__ __forceinline__ void block_total32(const Dev &d, int fi, int kind, fl
         const int nw = (int)(blockDim.x >> 5);
         df s{0.f, 0.f};
         for (int q = 0; q < nw; ++q) s = df_add_f(s, ws[q * NV + i]);
-        xsum_add(xsum_words(d, fi, kind) + (blockIdx.x % XSUM_COPIES) * (8 * XSUM_W) + i * XSUM_W,
-                 threadIdx.x < NV ? s.h : s.l);
+        xsum_add(xsum_words(d, fi, kind) + i * XSUM_W, threadIdx.x < NV ? s.h : s.l);
     }
     __syncthreads();
 }
 
-// In the last block: film fi's totals of the NV values, valid in thread 0.
+// What the last block of a film's pass works with, in shared memory: the
+// film's solver slot and the step counters as they were before the pass, and
+// the pass's totals.
+struct FilmTail {
+    SolveDev S;
+    Ctl c;
+    double tot[8];
+    int any;
+};
+
+// In the last block: film fi's totals of NV values (T.tot), its slot and the
+// counters, every word in one round trip; valid in every thread.  The
+// accumulators are cleared for the next pass.  A digit is below 2^53 for less
+// than 2^20 blocks, so the digits convert exactly and Horner's rule rounds
+// only what the leading 53 bits leave (no cancellation past one bit).
+// The tail of a pass runs once, on one SM whose instruction cache does not
+// hold it, at some 110 cycles per 8 instructions: a short rolled loop beats an
+// unrolled carry and rounding by a lane per digit (1.5 k against 5.5 k cycles
+// for the digits), and the whole tail of a TDGL step took 13.5 k cycles as
+// chains of dependent loads, FP64 divisions and long scalar code.
 template <int NV>
-__device__ __forceinline__ void film_total32(const Dev &d, int fi, int kind, double (&out)[NV])
+__device__ __forceinline__ void film_tail(const Dev &d, int fi, int kind, FilmTail &T)
 {
+    static_assert(NV * XSUM_W <= 128, "a thread per word");
     __shared__ long long s_w[NV * XSUM_W];
-    __shared__ double s_tot[NV];
-    if (threadIdx.x < NV * XSUM_W) {                // every word in one round trip; cleared for the next pass
-        unsigned long long *w = xsum_words(d, fi, kind) + threadIdx.x, c[XSUM_COPIES], t = 0ull;
-        #pragma unroll
-        for (int q = 0; q < XSUM_COPIES; ++q) c[q] = __ldcg(w + q * (8 * XSUM_W));
-        #pragma unroll
-        for (int q = 0; q < XSUM_COPIES; ++q) {
-            t += c[q];
-            __stcg(w + q * (8 * XSUM_W), 0ull);
-        }
-        s_w[threadIdx.x] = (long long)t;
+    const int t = threadIdx.x;
+    if (t < NV * XSUM_W) {
+        unsigned long long *w = xsum_words(d, fi, kind) + t;
+        s_w[t] = (long long)__ldcg(w);
+        __stcg(w, 0ull);
     }
+    #pragma unroll 1
+    for (int w = t; w < (int)(sizeof(SolveDev) / 4); w += blockDim.x) ((int *)&T.S)[w] = __ldcg((const int *)(d.solve + fi) + w);
+    if (t < (int)(sizeof(Ctl) / 4)) ((int *)&T.c)[t] = __ldcg((const int *)d.ctl + t);
     __syncthreads();
-    if (threadIdx.x < NV) s_tot[threadIdx.x] = xsum_value(s_w + threadIdx.x * XSUM_W);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        #pragma unroll
-        for (int i = 0; i < NV; ++i) out[i] = s_tot[i];
+    if (t < NV) {
+        const long long *c = s_w + t * XSUM_W;
+        double v = c[9] ? __longlong_as_double(0x7ff8000000000000ll) : 0.0;
+        #pragma unroll 1
+        for (int i = 8; i >= 0; --i) v = fma(v, 4294967296.0, (double)c[i]);
+        T.tot[t] = v * 1.401298464324817e-45;       // 2^-149
     }
     __syncthreads();
 }
+
+// A double is finite / positive, without the FP64 pipe.
+__device__ __forceinline__ bool fin64(double v) { return ((unsigned)__double2hiint(v) & 0x7ff00000u) != 0x7ff00000u; }
 
 // Block-uniform read of a flag another block may have written.
 __device__ __forceinline__ bool uniform_flag(const int *p)
@@ -644,25 +626,15 @@ __global__ void __launch_bounds__(NT) k_tdgl(Dev d, Fields<T> F)
 // Last block of a TDGL step: every film's sweep row from its items' partial
 // sums (evolve.cu:256-357 scaled as in :391-400), and the per-step reset of
 // the solver state.
-// Film fi's sweep row frow from the totals of its seven row sums (one thread).
-template <int NV>
-__device__ __forceinline__ void row_write(const Dev &d, int fi, int frow, const double (&sTot)[NV])
+// Film fi's sweep row frow from the totals of its seven row sums (thread q < 11
+// the row's value q; FilmDev::rowc: 1 / voxels, fractions); step: steps done.
+__device__ __forceinline__ void row_write(const Dev &d, int fi, int frow, const double *tot, int step)
 {
-    const FilmDev *ff = d.films + fi;
-    double *R = d.rowbuf + ((long long)fi * d.rstride + frow) * 11;
-    const double N = (double)ff->nx * ff->ny * ff->nz;
-    R[0] = sTot[0] * ff->inv_N;
-    R[1] = sTot[1] * ff->inv_N;
-    R[2] = sTot[2] * ff->inv_N;
-    R[3] = sTot[3] * ff->inv_N;
-    const double nFE = ff->n_mat[1], nAFE = ff->n_mat[0], nDE = ff->n_mat[2];
-    R[4] = nFE > 0.0 ? sTot[4] / nFE : 0.0;
-    R[5] = nFE > 0.0 ? nFE / N : 0.0;
-    R[6] = nAFE > 0.0 ? sTot[5] / nAFE : 0.0;
-    R[7] = nAFE > 0.0 ? nAFE / N : 0.0;
-    R[8] = nDE > 0.0 ? sTot[6] / nDE : 0.0;
-    R[9] = nDE > 0.0 ? nDE / N : 0.0;
-    R[10] = (double)(d.ctl->step + 1);
+    const int q = threadIdx.x;
+    if (q >= 11) return;
+    const double c = d.films[fi].rowc[q];
+    const int src = q < 5 ? q : q == 6 ? 5 : q == 8 ? 6 : -1;
+    d.rowbuf[((long long)fi * d.rstride + frow) * 11 + q] = q == 10 ? (double)(step + 1) : src >= 0 ? tot[src] * c : c;
 }
 
 // Film fi's solver state at the start of a step (one thread).
@@ -692,14 +664,15 @@ __device__ __forceinline__ void step_reopen(const Dev &d)
 // The FP32 TDGL step's end (finish32): film fi's sweep row and the reset of
 // its solver state; then the step's conditions.  Under kernel timing
 // (d.force) the totals are formed as a step forms them and nothing is written.
-__device__ __forceinline__ void tdgl_film32(const Dev &d, int rs, int fi, double (&sTot)[7])
+__device__ __forceinline__ void tdgl_film32(const Dev &d, int rs, int fi, FilmTail &T)
 {
     const int frow = d.rows[(long long)fi * d.wstride + rs];
     if (frow >= 0) {
-        film_total32<7>(d, fi, 0, sTot);
-        if (threadIdx.x == 0 && !d.force) row_write(d, fi, frow, sTot);
+        film_tail<7>(d, fi, 0, T);
+        if (!d.force) row_write(d, fi, frow, T.tot, T.c.step);
     }
     if (threadIdx.x == 0 && !d.force) step_reset(d, fi);
+    __syncthreads();                              // T is the next film's
 }
 __device__ __forceinline__ void tdgl_grid32(const Dev &d, int rs)
 {
@@ -718,7 +691,7 @@ __device__ __forceinline__ void tdgl_finish(const Dev &d, int rs, double (*sRed)
         const int frow = d.rows[(long long)fi * d.wstride + rs];
         if (frow >= 0) {
             film_total<7>(d, ff, sRed, sTot);
-            if (threadIdx.x == 0 && !d.force) row_write(d, fi, frow, sTot);
+            if (!d.force) row_write(d, fi, frow, sTot, d.ctl->step);
         }
         if (threadIdx.x == 0 && !d.force) step_reset(d, fi);
     }
@@ -902,89 +875,127 @@ __device__ __forceinline__ void step_end(const Dev &d)
 // ||r|| <= refine_tol ||b||, rotates the buffers and sets the next inner
 // solve's target.
 // Film fi's part (finish32): its totals, the stop test and its next pass.
-__device__ __forceinline__ void refine_film(const Dev &d, int fi, double (&sTot)[3])
+// T.S takes the outcome too.
+__device__ __forceinline__ void refine_film(const Dev &d, int fi, FilmTail &T)
 {
-    if (d.force) {              // kernel timing: the totals as a pass forms them; the state stays as it is
-        if (d.films[fi].dep_flag) film_total32<3>(d, fi, 1, sTot);
-        return;
-    }
-    {
-        const FilmDev *ff = d.films + fi;
+    const FilmDev *ff = d.films + fi;
+    // constants of the stop test, loaded with the totals
+    const double tol2 = ff->refine_tol2;
+    const int dep = ff->dep_flag, upd_ok = ff->upd_ok, defer_ok = ff->defer_ok, max_refine = ff->max_refine;
+    const int direct = ff->direct, inner_max = ff->inner_max;
+    const float dl = ff->cheb_delta;
+    if (!dep) return;
+    film_tail<3>(d, fi, 1, T);
+    if (threadIdx.x == 0 && !d.force && T.S.outer_active) {       // kernel timing: the state stays as it is
+        const SolveDev P = T.S;
         SolveDev *S = d.solve + fi;
-        const bool was = ff->dep_flag != 0 && uniform_flag(&S->outer_active);
-        if (was) film_total32<3>(d, fi, 1, sTot);
-        if (threadIdx.x == 0 && was) {
-            // an update pass (r <- r - A dx) leaves b.b as the last full pass formed it
-            const bool was_upd = ff->upd_ok && S->upd && S->refine > 0;
-            const double bb = was_upd ? S->bb : sTot[1];
-            const int c0 = S->phi_cur, p0 = S->phi_prev, q0 = S->phi_prev2, r0 = S->phi_prev3;
-            const int fr = 10 - c0 - p0 - q0 - r0;
-            const bool first = S->refine == 0;
-            if (first) {                     // keep phi_n .. phi_{n-2} for the next step's extrapolation
-                S->phi_prev3 = q0;
-                S->phi_prev2 = p0;
-                S->phi_prev = c0;
-                S->hist = min(S->hist + 1, 4);   // this step's potential joins the history
-                (void)r0;                    // phi_{n-3} is no longer needed: it becomes the free buffer
-            }
-            S->phi_cur = fr;                 // this pass wrote the free buffer
-            S->refine += 1;
-            S->rr64 = sTot[0];
-            S->bb = bb;
-            const bool conv = sTot[0] <= ff->refine_tol2 * bb || sTot[0] == 0.0;
-            // the next pass may update r when this one formed it in full and
-            // ||r|| <= 1e-4 ||b||: the FP32 rounding of A dx (relative ~1e-7,
-            // times the stencil's cancellation) then stays far below the
-            // refinement target; never two update passes in a row
-            S->upd = !was_upd && ff->upd_ok && sTot[0] <= 1e-8 * bb;
-            // the next direct solve's increment (Chebyshev semi-iteration for a
-            // direct solve preconditioning several eps, M^-1 A's spectrum in
-            // [1 - delta, 1 + delta]): solve 0 of a step dx = M^-1 r, then
-            // rho_k = 1 / (2 / delta - rho_{k-1}), dx_k = (2 rho_k / delta) M^-1 r
-            // + rho_k rho_{k-1} dx_{k-1}
-            {
-                const double dl = ff->cheb_delta;
-                if (dl <= 0.0 || S->refine == 1) {
-                    S->cheb_rho = dl;
-                    S->cheb_w = 1.f;
-                    S->cheb_m = 0.f;
-                } else {
-                    const double rp = S->cheb_rho, rk = 1.0 / (2.0 / dl - rp);
-                    S->cheb_rho = rk;
-                    S->cheb_w = (float)(2.0 * rk / dl);
-                    S->cheb_m = (float)(rk * rp);
-                }
-            }
-            S->iters = 0;
-            S->rz = S->rz0 = sTot[2];
-            if (conv || !isfinite(sTot[0])) {
-                S->outer_active = 0;
-                S->active = 0;
-                if (!isfinite(sTot[0])) S->status = 2;
-            } else if (S->refine > ff->max_refine) {
-                S->outer_active = 0;
-                S->active = 0;
-                S->status = 3;
-            } else {
-                S->active = isfinite(S->rz) && S->rz > 0.0;
-                if (!S->active) { S->outer_active = 0; S->status = 2; }
+        const double rr = T.tot[0], rz = T.tot[2];
+        // an update pass (r <- r - A dx) leaves b.b as the last full pass formed it
+        const bool was_upd = upd_ok && P.upd && P.refine > 0;
+        const double bb = was_upd ? P.bb : T.tot[1];
+        const int fr = 10 - P.phi_cur - P.phi_prev - P.phi_prev2 - P.phi_prev3;
+        const bool first = P.refine == 0;
+        if (first) {                     // keep phi_n .. phi_{n-2} for the next step's extrapolation;
+            S->phi_prev3 = P.phi_prev2;  // phi_{n-3} is no longer needed: it becomes the free buffer
+            S->phi_prev2 = P.phi_prev;
+            S->phi_prev = P.phi_cur;
+            S->hist = min(P.hist + 1, 4);    // this step's potential joins the history
+        }
+        S->phi_cur = fr;                 // this pass wrote the free buffer
+        const int refine = P.refine + 1;
+        S->refine = refine;
+        S->rr64 = rr;
+        S->bb = bb;
+        const bool fin = fin64(rr);
+        const bool conv = fin && (rr <= tol2 * bb || rr == 0.0);
+        // the next pass may update r when this one formed it in full and
+        // ||r|| <= 1e-4 ||b||: the FP32 rounding of A dx (relative ~1e-7,
+        // times the stencil's cancellation) then stays far below the
+        // refinement target; never two update passes in a row
+        const int upd = !was_upd && upd_ok && rr <= 1e-8 * bb;
+        S->upd = upd;
+        // the next direct solve's increment (Chebyshev semi-iteration for a
+        // direct solve preconditioning several eps, M^-1 A's spectrum in
+        // [1 - delta, 1 + delta]): solve 0 of a step dx = M^-1 r, then
+        // rho_k = 1 / (2 / delta - rho_{k-1}), dx_k = (2 rho_k / delta) M^-1 r
+        // + rho_k rho_{k-1} dx_{k-1} (weights of FP32 increments, in FP32)
+        if (dl <= 0.f || refine == 1) {
+            S->cheb_rho = dl;
+            S->cheb_w = 1.f;
+            S->cheb_m = 0.f;
+        } else {
+            const float rp = P.cheb_rho, rk = 1.f / (2.f / dl - rp);
+            S->cheb_rho = rk;
+            S->cheb_w = 2.f * rk / dl;
+            S->cheb_m = rk * rp;
+        }
+        S->iters = 0;
+        S->rz = S->rz0 = rz;
+        int outer = 1, active = 0;
+        if (conv || !fin) {
+            outer = 0;
+            if (!fin) S->status = 2;
+        } else if (refine > max_refine) {
+            outer = 0;
+            S->status = 3;
+        } else {
+            active = fin64(rz) && rz > 0.0;
+            if (!active) { outer = 0; S->status = 2; }
+            if (!direct) {
                 // inner target: just enough reduction to reach the refinement
                 // tolerance in this pass (half-margin), between the FP32 floor
                 // inner_tol and 1e-2
-                double want = 0.25 * ff->refine_tol2 * bb / sTot[0];
+                double want = 0.25 * tol2 * bb / rr;
                 want = fmax(want, ff->inner_tol2);
                 S->inner_tol2 = fmin(want, 1e-4);
-                S->inner_max = ff->inner_max;
-                // the step's first pass before an exact direct solve: the step
-                // ends on that solve, and the next TDGL step forms the check
-                // the update pass would have formed (SolveDev::pending)
-                if (d.defer && ff->defer_ok && first && S->upd && S->active) {
-                    S->pending = 1;
-                    S->outer_active = 0;
-                }
+                S->inner_max = inner_max;
+            }
+            // the step's first pass before an exact direct solve: the step
+            // ends on that solve, and the next TDGL step forms the check
+            // the update pass would have formed (SolveDev::pending)
+            if (d.defer && defer_ok && first && upd && active) {
+                S->pending = 1;
+                T.S.pending = 1;
+                outer = 0;
             }
         }
+        S->outer_active = outer;
+        S->active = active;
+        T.S.outer_active = outer;
+        T.S.active = active;
+        T.S.refine = refine;
+        T.S.status = (conv || fin) ? T.S.status : 2;
+        if (!conv && fin && refine > max_refine) T.S.status = 3;
+        if (!conv && fin && refine <= max_refine && !active) T.S.status = 2;
     }
+    __syncthreads();
+}
+
+// The end of a time step of a single film (thread 0), from its slot and the
+// counters in shared memory.
+__device__ __forceinline__ void step_end1(const Dev &d, const FilmTail &T)
+{
+    const SolveDev &S = T.S;
+    d.iters_log[T.c.run_step] = S.total_iters;
+    d.refine_log[T.c.run_step] = S.refine + (S.pending ? 1 : 0);
+    if (S.status != 0 && S.status != 3 && S.sticky == 0) d.solve->sticky = S.status;
+    d.ctl->step = T.c.step + 1;
+    d.ctl->run_step = T.c.run_step + 1;
+    d.ctl->cur = T.c.cur ^ 1;
+}
+
+// The same for a single film, from T.
+__device__ __forceinline__ void refine_grid1(const Dev &d, FilmTail &T)
+{
+    if (threadIdx.x != 0) return;
+    if (!d.force) {
+        const int outer = d.films->dep_flag ? T.S.outer_active : 0;
+        set_cond(d, d.h_outer, outer);
+        set_cond(d, d.h_inner, d.films->dep_flag ? T.S.active : 0);
+        if (d.arrive) *d.arrive = 0u;
+        if (d.step_end && !outer) step_end1(d, T);
+    }
+    *d.counter = 0u;
 }
 
 // What depends on every film (finish32): the loop conditions, and the end of

@@ -417,6 +417,24 @@ __device__ __forceinline__ bool spec_run(const Dev &d, int f)
 // films all end on this solve ends here.
 __device__ __forceinline__ void spec_end(const Dev &d)
 {
+    if (d.n_films == 1) {
+        // the slot and the counters in one round trip
+        __shared__ FilmTail T;
+        for (int w = threadIdx.x; w < (int)(sizeof(SolveDev) / 4); w += blockDim.x) ((int *)&T.S)[w] = __ldcg((const int *)d.solve + w);
+        if (threadIdx.x < sizeof(Ctl) / 4) ((int *)&T.c)[threadIdx.x] = __ldcg((const int *)d.ctl + threadIdx.x);
+        __syncthreads();
+        if (threadIdx.x != 0) return;
+        *d.counter = 0u;
+        if (d.force) return;
+        if (T.S.active) {
+            T.S.total_iters += 1;
+            d.solve->iters = 1;
+            d.solve->total_iters = T.S.total_iters;
+            d.solve->active = 0;
+        }
+        if (d.defer && d.step_end && !T.S.outer_active) step_end1(d, T);
+        return;
+    }
     __shared__ int s_out;
     if (threadIdx.x == 0) {
         int out = 0;

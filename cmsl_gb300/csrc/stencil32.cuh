@@ -295,9 +295,9 @@ template <int TYc, bool DEF = false> constexpr size_t t32_smem()
     return sizeof(float) * T32_NS * t32_stage<TYc, DEF>();
 }
 
-template <int NV>
-__device__ __forceinline__ void tdgl_def_film(const Dev &d, int rs, int fi, double (&sTot)[NV]);
+__device__ __forceinline__ void tdgl_def_film(const Dev &d, int rs, int fi, FilmTail &T);
 __device__ __forceinline__ void tdgl_def_grid(const Dev &d, int rs);
+__device__ __forceinline__ void tdgl_def_grid1(const Dev &d, int rs, FilmTail &T);
 
 // TYc: the tile height (TX x TYc threads, one column each).
 // DEF: a film whose previous step ended on its direct solve (SolveDev::pending;
@@ -328,7 +328,7 @@ __global__ void __launch_bounds__(TileShape<TYc>::NTt, tdgl32_minb<TYc, DEF>()) 
     float *ring = (float *)smem_t32;
     __shared__ float4 sC[6][3];
     __shared__ double sRed[NT / 32][NV];
-    __shared__ double sTot[NV];
+    __shared__ FilmTail tail;
     const int4 it = d.sitems[blockIdx.x];
     const FilmDev *f = d.films + it.x;
     const int z0 = it.w & 0xffff, z1 = it.w >> 16;
@@ -472,9 +472,10 @@ __global__ void __launch_bounds__(TileShape<TYc>::NTt, tdgl32_minb<TYc, DEF>()) 
 
     if (row >= 0 || pend) block_total32<NV>(d, it.x, 0, acc, sRed);
     if constexpr (DEF)
-        finish32<FB>(d, [&](int fi) { tdgl_def_film<NV>(d, rs, fi, sTot); }, [&] { tdgl_def_grid(d, rs); });
+        finish32<FB>(d, [&](int fi) { tdgl_def_film(d, rs, fi, tail); },
+                     [&] { if (FB) tdgl_def_grid(d, rs); else tdgl_def_grid1(d, rs, tail); });
     else
-        finish32<FB>(d, [&](int fi) { tdgl_film32(d, rs, fi, sTot); }, [&] { tdgl_grid32(d, rs); });
+        finish32<FB>(d, [&](int fi) { tdgl_film32(d, rs, fi, tail); }, [&] { tdgl_grid32(d, rs); });
 }
 
 // The end of a TDGL step that may carry deferred checks (finish32): every
@@ -488,24 +489,16 @@ __global__ void __launch_bounds__(TileShape<TYc>::NTt, tdgl32_minb<TYc, DEF>()) 
 // the same result), and the step loop runs this step again after that pass
 // has ended the previous one.
 // Film fi's part: its sweep row and its check's r.r (S->rr64).
-template <int NV>
-__device__ __forceinline__ void tdgl_def_film(const Dev &d, int rs, int fi, double (&sTot)[NV])
+__device__ __forceinline__ void tdgl_def_film(const Dev &d, int rs, int fi, FilmTail &T)
 {
-    static_assert(NV == 8, "seven row sums and the check's r.r");
     const FilmDev *ff = d.films + fi;
-    SolveDev *S = d.solve + fi;
-    const int frow = d.rows[(long long)fi * d.wstride + rs];
-    if (d.force) {              // kernel timing: the totals as a step forms them; the state stays as it is
-        if (ff->dep_flag || frow >= 0) film_total32<NV>(d, fi, 0, sTot);
-        return;
+    const int frow = d.rows[(long long)fi * d.wstride + rs], dep = ff->dep_flag;
+    film_tail<8>(d, fi, 0, T);
+    if (!d.force) {             // kernel timing: the totals as a step forms them; the state stays as it is
+        if (frow >= 0) row_write(d, fi, frow, T.tot, T.c.step);
+        if (threadIdx.x == 0 && dep && T.S.pending) d.solve[fi].rr64 = T.tot[7];
     }
-    const bool pend = ff->dep_flag != 0 && uniform_flag(&S->pending);
-    if (frow < 0 && !pend) return;
-    film_total32<NV>(d, fi, 0, sTot);
-    if (threadIdx.x == 0) {
-        if (frow >= 0) row_write(d, fi, frow, sTot);
-        if (pend) S->rr64 = sTot[NV - 1];
-    }
+    __syncthreads();            // T is the next film's
 }
 
 // A pending film's check passed (NaN fails); rr read past this block's L1.
@@ -554,6 +547,41 @@ __device__ __forceinline__ void tdgl_def_grid(const Dev &d, int rs)
         }
         step_reopen(d);
         set_cond(d, d.h_steps, 1);
+    }
+    *d.counter = 0u;
+}
+
+// The same for a single film, from its tail T (thread 0): the slot's fields
+// are at hand, so the step begins or reopens with stores alone.
+__device__ __forceinline__ void tdgl_def_grid1(const Dev &d, int rs, FilmTail &T)
+{
+    if (threadIdx.x != 0) return;
+    if (!d.force) {
+        SolveDev *S = d.solve;
+        const FilmDev *f = d.films;
+        const double rr = T.tot[7];
+        const bool pend = f->dep_flag && T.S.pending;
+        const bool ok = rr <= f->refine_tol2 * T.S.bb || rr == 0.0;
+        if (!pend || ok) {
+            if (T.S.pending) {
+                // this launch wrote x0 + dx to the free buffer; the warm start
+                // buffer (x0) takes the third-oldest slot, which held the next
+                // warm start and now becomes the free one
+                S->phi_prev3 = T.S.phi_cur;
+                S->phi_cur = 10 - T.S.phi_cur - T.S.phi_prev - T.S.phi_prev2 - T.S.phi_prev3;
+                S->pending = 0;
+            }
+            step_reset(d, 0);
+            step_begin(d, rs);
+        } else {
+            S->pending = 0;
+            S->outer_active = 1;
+            S->active = 0;
+            S->refine = 1;
+            S->upd = 1;
+            step_reopen(d);
+            set_cond(d, d.h_steps, 1);
+        }
     }
     *d.counter = 0u;
 }
@@ -699,7 +727,7 @@ __global__ void __launch_bounds__(TileShape<TYc>::NTt, TileShape<TYc>::MINB) k_r
     extern __shared__ float4 smem_r32[];
     float *ring = (float *)smem_r32;
     __shared__ double sRed[NT / 32][3];
-    __shared__ double sTot[3];
+    __shared__ FilmTail tail;
     const int4 it = d.sitems[blockIdx.x];
     const FilmDev *f = d.films + it.x;
     const SolveDev *S = d.solve + it.x;
@@ -813,7 +841,7 @@ __global__ void __launch_bounds__(TileShape<TYc>::NTt, TileShape<TYc>::MINB) k_r
     }
     cp_wait<0>();
     if (run) block_total32<3>(d, it.x, 1, acc, sRed);
-    finish32<FB>(d, [&](int fi) { refine_film(d, fi, sTot); }, [&] { refine_grid(d); });
+    finish32<FB>(d, [&](int fi) { refine_film(d, fi, tail); }, [&] { if (FB) refine_grid(d); else refine_grid1(d, tail); });
 }
 
 }  // namespace cmsl

@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(NT, 4) k_tdgl32t(Dev d, Fields<float> F)
     __shared__ TmaOp ops[TT_OPS];
     __shared__ float4 sC[6][3];
     __shared__ double sRed[NT / 32][7];
-    __shared__ double sTot[7];
+    __shared__ FilmTail tail;
     const int4 it = d.sitems[blockIdx.x];
     const FilmDev *f = d.films + it.x;
     const int z0 = it.w & 0xffff, z1 = it.w >> 16;
@@ -255,7 +255,7 @@ __global__ void __launch_bounds__(NT, 4) k_tdgl32t(Dev d, Fields<float> F)
     }
 
     if (row >= 0) block_total32<7>(d, it.x, 0, acc, sRed);
-    finish32<FB>(d, [&](int fi) { tdgl_film32(d, rs, fi, sTot); }, [&] { tdgl_grid32(d, rs); });
+    finish32<FB>(d, [&](int fi) { tdgl_film32(d, rs, fi, tail); }, [&] { tdgl_grid32(d, rs); });
 }
 
 // ------------------------------------------------- double-float residual
@@ -281,7 +281,7 @@ __global__ void __launch_bounds__(NT, 4) k_refine32t(Dev d, Fields<float> F)
     __shared__ __align__(8) uint64_t bar[NS];
     __shared__ TmaOp ops[RT_OPS];
     __shared__ double sRed[NT / 32][3];
-    __shared__ double sTot[3];
+    __shared__ FilmTail tail;
     const int4 it = d.sitems[blockIdx.x];
     const FilmDev *f = d.films + it.x;
     const SolveDev *S = d.solve + it.x;
@@ -384,7 +384,7 @@ __global__ void __launch_bounds__(NT, 4) k_refine32t(Dev d, Fields<float> F)
         if (apply) nh[o] = make_float2(c.xc.h, c.xc.l);
     }
     if (run) block_total32<3>(d, it.x, 1, acc, sRed);
-    finish32<FB>(d, [&](int fi) { refine_film(d, fi, sTot); }, [&] { refine_grid(d); });
+    finish32<FB>(d, [&](int fi) { refine_film(d, fi, tail); }, [&] { if (FB) refine_grid(d); else refine_grid1(d, tail); });
 }
 
 
