@@ -26,6 +26,7 @@
 // step loop's condition compares with the run's length.
 #include <algorithm>
 #include <cmath>
+#include <complex>
 #include <cstdarg>
 #include <cstdio>
 #include <cstdlib>
@@ -193,6 +194,14 @@ std::string shape_key(const Engine *e)
     return k;
 }
 
+constexpr int SPEC_CHIRP_MAX = 2048;        // longest chirp transform: through 4096 values
+// Columns from which AUTO takes the direct solve at sides other than 2^a 3^b.
+// It is the faster one at every size measured (a step 33x32x6 207 -> 67 us,
+// 50x50x10 313 -> 79, 150x110x21 820 -> 96, 317x311x21 1627 -> 350, 500x500x32
+// 8838 -> 878); smaller films keep the PCG, which is what
+// cmsl_film_inner_solver has always answered for them.
+constexpr long long SPEC_CHIRP_COLUMNS = 1024;
+
 // n = 2^a 3^b <= 4096 (the FFT radices of spectral.cuh)
 bool spec_radix_ok(int n)
 {
@@ -202,12 +211,45 @@ bool spec_radix_ok(int n)
     return n == 1;
 }
 
+// The tables of a chirp transform of length n through m = 2^lgm, appended to
+// tw: w_j = exp(-i pi j^2 / n), the transform of conj(w) around zero over m
+// (with the 1 / m of the inverse), the m twiddles.  In double.
+void spec_chirp_tables(int n, int lgm, std::vector<float2> &tw)
+{
+    const int m = 1 << lgm;
+    std::vector<std::complex<double>> c((size_t)m), t((size_t)m);
+    auto put = [&](std::complex<double> v) { tw.push_back(make_float2((float)v.real(), (float)v.imag())); };
+    for (int j = 0; j < n; ++j) {
+        const std::complex<double> w = std::polar(1.0, -M_PI * (double)((long long)j * j % (2ll * n)) / n);
+        put(w);
+        c[j] = std::conj(w);
+        if (j) c[m - j] = std::conj(w);
+    }
+    for (int len = m, s = 1; len > 1; len /= 2, s *= 2) {           // Stockham radix-2 passes
+        for (int p = 0; p < len / 2; ++p) {
+            const std::complex<double> w = std::polar(1.0, -2.0 * M_PI * p / len);
+            for (int q = 0; q < s; ++q) {
+                const auto x = c[q + s * p], y = c[q + s * (p + len / 2)];
+                t[q + s * 2 * p] = x + y;
+                t[q + s * (2 * p + 1)] = (x - y) * w;
+            }
+        }
+        c.swap(t);
+    }
+    for (int j = 0; j < m; ++j) put(c[j] / (double)m);
+    for (int j = 0; j < m; ++j) put(std::polar(1.0, -2.0 * M_PI * j / m));
+}
+
 SpecAxis spec_plan(int n)
 {
     SpecAxis a{};
     a.n = n;
     a.lg = (n & (n - 1)) == 0 ? __builtin_ctz((unsigned)n) : -1;
     if (a.lg >= 0) return a;
+    if (!spec_radix_ok(n)) {
+        while ((1 << a.lgm) < 2 * n - 1) ++a.lgm;
+        return a;
+    }
     // the fewest passes; the radices as even as they can be (the least largest
     // one), so that every pass has butterflies for most threads
     static const int R[] = {16, 12, 9, 8, 6, 4, 3, 2};
@@ -1332,12 +1374,13 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
         all_uni &= descs[i].mats[0].eps_r == descs[i].mats[1].eps_r && descs[i].mats[1].eps_r == descs[i].mats[2].eps_r;
     }
     // direct (spectral) inner solve: every film with a depolarisation solve
-    // has the Dirichlet z boundary and 2^a 3^b sides; with one eps it is the
+    // has 2^a 3^b sides or, under AUTO, others that the chirp transforms take
+    // (DIRECT also asks for the Dirichlet z boundary); with one eps it is the
     // exact inverse, with several a preconditioner of the refinement
     int spec_mmax = 1;
     {
         bool want = false, forced = false, ok = e->precision != CMSL_FP64, anydep = false, ok_auto = true;
-        bool dirichlet = true;
+        bool dirichlet = true, fast = true, chirp = true;
         for (int i = 0; i < n; ++i) {
             const cmsl_film_desc &d = descs[i];
             forced |= d.inner_solver == CMSL_INNER_DIRECT;
@@ -1349,15 +1392,18 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
             // several permittivities: the solve preconditions the refinement
             // (AUTO up to SPEC_PRECOND_KAPPA, any ratio when DIRECT is asked for)
             ok_auto &= kappa <= SPEC_PRECOND_KAPPA;
-            ok &= d.nz >= 3 && spec_radix_ok(d.nx) && spec_radix_ok(d.ny);
+            ok &= d.nz >= 3;
+            fast &= spec_radix_ok(d.nx) && spec_radix_ok(d.ny);
+            for (int side : {d.nx, d.ny}) chirp &= spec_radix_ok(side) || (side > 1 && side <= SPEC_CHIRP_MAX);
+            chirp &= (long long)d.nx * d.ny >= SPEC_CHIRP_COLUMNS || (spec_radix_ok(d.nx) && spec_radix_ok(d.ny));
             dirichlet &= d.zbc == CMSL_DIRICHLET;
             spec_mmax = std::max(spec_mmax, d.zbc == CMSL_DIRICHLET ? d.nz - 2 : d.nz);
         }
         ok &= anydep && spec_zthreads(spec_mmax) > 0;
-        if (forced && !(ok && dirichlet))
+        if (forced && !(ok && fast && dirichlet))
             return fail(CMSL_ERR_ARG, "inner_solver DIRECT needs FP32_REFINED films whose depolarisation solves have "
                                       "the Dirichlet z boundary and nx, ny of the form 2^a 3^b <= 4096");
-        e->spectral = ok && want && (forced || ok_auto);
+        e->spectral = ok && want && (forced || (ok_auto && chirp));
     }
     int cg_per = 0, cg_nsm = 0;
     e->persistent = e->precision != CMSL_FP64 && !e->spectral && all_dirichlet && n <= CG_MAX_FILMS &&
@@ -1649,6 +1695,7 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
         std::vector<float> lam;
         long long coff = 0;
         size_t smx = 0, smy = 0;
+        bool chirp = false;                                         // a chirp transform among the films
         auto tables = [&](int nn, int *two, int *lamo) {
             *two = (int)tw.size();
             *lamo = (int)lam.size();
@@ -1687,6 +1734,12 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
             P.scale = (float)(h.h * h.h / (eps * (double)h.nx * h.ny));
             tables(h.nx, &P.twx, &P.lamx);
             tables(h.ny, &P.twy, &P.lamy);
+            for (SpecAxis *ax : {&P.ax, &P.ay})
+                if (ax->lgm) {
+                    ax->ch = (int)tw.size();
+                    spec_chirp_tables(ax->n, ax->lgm, tw);
+                }
+            chirp |= P.ax.lgm || P.ay.lgm;
             // rows (columns) per transform block: about two blocks per SM for
             // the film's Mp ny rows (Mp nx columns), a power of two, at most
             // SPEC_ELEMS values (8 rows of 256 at 256x256x32, 8 of 512 at
@@ -1699,7 +1752,8 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
                 if (rbe && atoi(rbe) > 0) r = std::min(cap, atoi(rbe));
                 return r;
             };
-            const int rbx = per_block((long long)P.Mp * h.ny, h.nx), cby = per_block((long long)P.Mp * h.nx, h.ny);
+            const int rbx = per_block((long long)P.Mp * h.ny, fft_len(P.ax)),
+                      cby = per_block((long long)P.Mp * h.nx, fft_len(P.ay));
             P.rb = rbx;
             P.cb = cby;
             const long long gx = ((long long)P.Mp * h.ny + rbx - 1) / rbx;
@@ -1715,8 +1769,9 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
                 smc = std::max(smc, spec_cl_bytes(h.nx, h.ny));
             }
             smq = std::max(smq, spec_yzy_bytes(h.ny, P.Mp, P.M));
-            smx = std::max(smx, sizeof(float2) * (2 * (spec_pad(rbx * spec_x_pitch(h.nx, true)) + 1) + h.nx));   // two tiles + twiddles
-            smy = std::max(smy, sizeof(float2) * (2 * cby * h.ny + h.ny));
+            const int lx = fft_len(P.ax), ly = fft_len(P.ay);
+            smx = std::max(smx, sizeof(float2) * (2 * (spec_pad(rbx * spec_x_pitch(lx, true)) + 1) + lx));   // two tiles + twiddles
+            smy = std::max(smy, sizeof(float2) * (2 * cby * ly + ly));
         }
         // the column layout (three launches per solve instead of five) where
         // the column pairs fit one block and every film has at most 128 x 128
@@ -1729,7 +1784,7 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
             for (int fi = 0; fi < n; ++fi) small = small && (long long)e->fh[fi].nx * e->fh[fi].ny <= 128 * 128;
             const char *cl = getenv("CMSL_SPEC_COLS");
             const bool want = cl && *cl ? atoi(cl) != 0 : small;
-            e->spec_col = e->spec_cl || (smq <= (size_t)optin && want);
+            e->spec_col = e->spec_cl || (smq <= (size_t)optin && want && !chirp);
         }
         // Thomas pivots of every film, mode and interior plane, in double:
         // dg = lam_x + lam_y + 2, inv_k = 1 / (dg - c'_{k-1}) with c'_k = -inv_k
@@ -1791,12 +1846,15 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
             bool mixed = false;
             for (int fi = 0; fi < n; ++fi) mixed |= e->fh[fi].dep && (sf[fi].ax.lg < 0 || sf[fi].ay.lg < 0);
             const bool col = e->spec_col && !e->spec_cl;
-            e->spec_x[0] = col ? mixed ? (void *)k_spec_x<true, true, true> : (void *)k_spec_x<true, true, false>
-                               : mixed ? (void *)k_spec_x<true, false, true> : (void *)k_spec_x<true, false, false>;
-            e->spec_x[1] = col ? mixed ? (void *)k_spec_x<false, true, true> : (void *)k_spec_x<false, true, false>
-                               : mixed ? (void *)k_spec_x<false, false, true> : (void *)k_spec_x<false, false, false>;
-            e->spec_y = mixed ? (void *)k_spec_y<true> : (void *)k_spec_y<false>;
-            e->spec_yzy = mixed ? (void *)k_spec_yzy<true> : (void *)k_spec_yzy<false>;
+            auto pick = [&](void *pow2, void *mix, void *any) { return chirp ? any : mixed ? mix : pow2; };
+            e->spec_x[0] = col ? mixed ? (void *)k_spec_x<true, true, FFT_MIXED> : (void *)k_spec_x<true, true, FFT_POW2>
+                               : pick((void *)k_spec_x<true, false, FFT_POW2>, (void *)k_spec_x<true, false, FFT_MIXED>,
+                                      (void *)k_spec_x<true, false, FFT_CHIRP>);
+            e->spec_x[1] = col ? mixed ? (void *)k_spec_x<false, true, FFT_MIXED> : (void *)k_spec_x<false, true, FFT_POW2>
+                               : pick((void *)k_spec_x<false, false, FFT_POW2>, (void *)k_spec_x<false, false, FFT_MIXED>,
+                                      (void *)k_spec_x<false, false, FFT_CHIRP>);
+            e->spec_y = pick((void *)k_spec_y<FFT_POW2>, (void *)k_spec_y<FFT_MIXED>, (void *)k_spec_y<FFT_CHIRP>);
+            e->spec_yzy = mixed ? (void *)k_spec_yzy<FFT_MIXED> : (void *)k_spec_yzy<FFT_POW2>;
             e->spec_grid[3] = (int)bqf.size();
             e->spec_smem[3] = smq;
             for (void *fn : e->spec_x)

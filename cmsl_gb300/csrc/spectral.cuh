@@ -20,7 +20,8 @@
 //
 // FFTs: self-sorting (Stockham) passes through shared memory, the butterflies
 // in registers -- radix 16 (8, 4 or 2 for the remainder) for powers of two,
-// the fewest radices up to 16 otherwise -- one block per group of rows (x) or of columns
+// the fewest radices up to 16 for 2^a 3^b, a chirp transform through powers of
+// two for any other length -- one block per group of rows (x) or of columns
 // (y); twiddles exp(-2 pi i t / n) and eigenvalues come from host tables
 // computed in double.  The z solve keeps the Thomas elimination in shared
 // memory, so each spectrum value is read and written once per sweep.
@@ -47,6 +48,8 @@ constexpr int SPEC_NT = 256;
 struct SpecAxis {
     int n, nst;
     int lg;                     // log2(n) when n is a power of two, else -1
+    int lgm;                    // lengths that are not 2^a 3^b: log2 of the chirp transform's length m >= 2 n - 1
+    int ch;                     // and its tables in SpecDev::tw: chirp [n], spectrum [m], twiddles [m]
     int rad[SPEC_MAX_STAGES];
 };
 
@@ -394,15 +397,71 @@ __device__ __forceinline__ void fft_mixed(float2 *a, float2 *b, int nseq, const 
     }
 }
 
-// The transform of nseq sequences along ax between ld and st.  MIXED: the
-// launch has films whose sides are no powers of two (a compile-time choice:
-// the radices of those cost the others' kernels registers).
-template <bool SEQ_FAST, bool MIXED, class LD, class ST>
-__device__ __forceinline__ void fft_any(float2 *a, float2 *b, int nseq, const SpecAxis &ax, int es, int ss,
-                                        const float2 *tw, LD ld, ST st)
+__device__ __forceinline__ int fft_pow2_passes(int lgn)
 {
-    if (!MIXED || ax.lg >= 0) fft_pow2<SEQ_FAST>(a, b, nseq, ax.lg, es, ss, tw, ld, st);
-    else if constexpr (MIXED) fft_mixed<SEQ_FAST>(a, b, nseq, ax, es, ss, tw, ld, st);
+    int n = 0;
+    for (int lgNs = 0; lgNs < lgn; ++n) {
+        const int rem = lgn - lgNs;
+        lgNs += (rem >= 4 && (rem & 3) != 1) ? 4 : rem >= 3 ? 3 : rem;
+    }
+    return n;
+}
+
+// Any other length n (Bluestein's chirp transform): with w_j = exp(-i pi j^2 / n),
+// X_k = w_k sum_j (x_j w_j) conj(w_(k-j)), a circular convolution of length
+// m = 2^lgm >= 2 n - 1 by two power-of-two transforms.  ch: the n values w_j,
+// then the transform of conj(w) over m (host tables formed in double).
+// The tiles hold m values per sequence, tw the m twiddles.  Four to eight
+// times the butterflies of a fast length, but at these sizes a transform is
+// launch and latency: a 150x110x21 film's step, whose PCG took some 65
+// iterations of 10 us, 820 -> 96 us.  Radices 5, 7, 11 would
+// only serve some lengths and cost every mixed kernel their registers.
+template <bool SEQ_FAST, class LD, class ST>
+__device__ __forceinline__ void fft_chirp(float2 *a, float2 *b, int nseq, int n, int lgm, int es, int ss,
+                                          const float2 *tw, const float2 *ch, LD ld, ST st)
+{
+    float2 *T = (fft_pow2_passes(lgm) & 1) == 0 ? a : b, *U = T == a ? b : a;
+    auto at = [&](int sq, int e) { return SEQ_FAST ? sq * ss + e * es : spec_pad(sq * ss + e * es); };
+    fft_pow2<SEQ_FAST>(a, b, nseq, lgm, es, ss, tw,
+                       [&](int sq, int e) { return e < n ? c_mul(ld(sq, e), __ldg(ch + e)) : make_float2(0.f, 0.f); },
+                       [&](int sq, int e, float2 v) {
+                           const float2 q = c_mul(v, __ldg(ch + n + e));
+                           T[at(sq, e)] = make_float2(q.x, -q.y);
+                       });
+    __syncthreads();
+    fft_pow2<SEQ_FAST>(T, U, nseq, lgm, es, ss, tw, [&](int sq, int e) { return T[at(sq, e)]; },
+                       [&](int sq, int e, float2 v) {
+                           if (e < n) st(sq, e, c_mul(make_float2(v.x, -v.y), __ldg(ch + e)));
+                       });
+}
+
+// The lengths among a launch's films (a compile-time choice: the other
+// radices and the chirp transform cost the kernels registers).
+enum { FFT_POW2 = 0, FFT_MIXED = 1, FFT_CHIRP = 2 };
+
+// The transform of nseq sequences along ax between ld and st.  tables:
+// SpecDev::tw.
+template <bool SEQ_FAST, int LEN, class LD, class ST>
+__device__ __forceinline__ void fft_any(float2 *a, float2 *b, int nseq, const SpecAxis &ax, int es, int ss,
+                                        const float2 *tw, const float2 *tables, LD ld, ST st)
+{
+    if (LEN == FFT_POW2 || ax.lg >= 0) fft_pow2<SEQ_FAST>(a, b, nseq, ax.lg, es, ss, tw, ld, st);
+    else if (LEN == FFT_MIXED || ax.lgm == 0) {
+        if constexpr (LEN != FFT_POW2) fft_mixed<SEQ_FAST>(a, b, nseq, ax, es, ss, tw, ld, st);
+    } else {
+        if constexpr (LEN == FFT_CHIRP) fft_chirp<SEQ_FAST>(a, b, nseq, ax.n, ax.lgm, es, ss, tw, tables + ax.ch, ld, st);
+    }
+}
+
+// Values per sequence of the tiles (and twiddles) of a transform along ax.
+__host__ __device__ __forceinline__ int fft_len(const SpecAxis &ax) { return ax.lgm ? 1 << ax.lgm : ax.n; }
+// Stages the twiddles of ax (twn: those of length n) in shared memory.
+template <int LEN>
+__device__ __forceinline__ void fft_twiddles(float2 *tw, const SpecAxis &ax, int twn, const float2 *tables)
+{
+    const int len = LEN == FFT_CHIRP ? fft_len(ax) : ax.n;
+    const float2 *src = tables + (LEN == FFT_CHIRP && ax.lgm ? ax.ch + ax.n + len : twn);
+    for (int t = threadIdx.x; t < len; t += blockDim.x) tw[t] = __ldg(src + t);
 }
 
 // Whether film f's inner solve runs through the spectra in this pass.
@@ -468,22 +527,12 @@ __device__ __forceinline__ void spec_finish(const Dev &d)
 // y.  Shared memory: two padded tiles of rb rows and the twiddles.
 __host__ __device__ inline int spec_x_pitch(int nx, bool col) { return col ? nx + 1 : nx; }
 
-__device__ __forceinline__ int fft_pow2_passes(int lgn)
+template <int LEN> __device__ __forceinline__ int fft_passes(const SpecAxis &ax)
 {
-    int n = 0;
-    for (int lgNs = 0; lgNs < lgn; ++n) {
-        const int rem = lgn - lgNs;
-        lgNs += (rem >= 4 && (rem & 3) != 1) ? 4 : rem >= 3 ? 3 : rem;
-    }
-    return n;
+    return LEN == FFT_POW2 || ax.lg >= 0 ? fft_pow2_passes(ax.lg) : ax.nst;
 }
 
-template <bool MIXED> __device__ __forceinline__ int fft_passes(const SpecAxis &ax)
-{
-    return !MIXED || ax.lg >= 0 ? fft_pow2_passes(ax.lg) : ax.nst;
-}
-
-template <bool IN_REAL, bool COL, bool MIXED>
+template <bool IN_REAL, bool COL, int LEN>
 __global__ void __launch_bounds__(SPEC_NT, 4) k_spec_x(Dev d, Fields<float> F, SpecDev sp)
 {
     extern __shared__ float2 sm2[];
@@ -504,10 +553,10 @@ __global__ void __launch_bounds__(SPEC_NT, 4) k_spec_x(Dev d, Fields<float> F, S
     // row pitch of the tiles: nx, or nx + 1 in the column layout, whose
     // transposed copies read a column of the tile (an odd pitch in 8-byte
     // words spreads its rows over the banks)
-    const int pitch = spec_x_pitch(nx, COL);
+    const int pitch = LEN == FFT_CHIRP ? fft_len(ax) : spec_x_pitch(nx, COL);
     const int tile = spec_pad(rb * pitch) + 1;
     float2 *a = sm2, *b = sm2 + tile, *tw = sm2 + 2 * tile;
-    for (int t = threadIdx.x; t < nx; t += blockDim.x) tw[t] = __ldg(sp.tw + P.twx + t);
+    fft_twiddles<LEN>(tw, ax, P.twx, sp.tw);
     // spectrum value (row r0 + sq, x element e) in the column layout
     auto col_at = [&](int sq, int e) -> long long {
         const int rw = r0 + sq, j = rw / ny;
@@ -531,7 +580,7 @@ __global__ void __launch_bounds__(SPEC_NT, 4) k_spec_x(Dev d, Fields<float> F, S
         return make_float2(rr[o], 2 * j + 1 < M ? rr[o + plane] : 0.f);
     };
     // the tile that receives the transform in the column layout's store
-    float2 *res = (fft_passes<MIXED>(ax) & 1) == 0 ? a : b;
+    float2 *res = (fft_passes<LEN>(ax) & 1) == 0 ? a : b;
     // the increment of this solve: w M^-1 r + m (the previous increment), from
     // the film's Chebyshev recurrence (w = 1, m = 0 for an exact solve)
     const SolveDev *Sf = d.solve + f;
@@ -559,7 +608,7 @@ __global__ void __launch_bounds__(SPEC_NT, 4) k_spec_x(Dev d, Fields<float> F, S
         }
     };
     __syncthreads();                                                     // twiddles
-    fft_any<false, MIXED>(a, b, nr, ax, 1, pitch, tw, ld, st);
+    fft_any<false, LEN>(a, b, nr, ax, 1, pitch, tw, sp.tw, ld, st);
     if (COL && IN_REAL) {
         // transposed store: consecutive threads write consecutive rows of one column
         __syncthreads();
@@ -574,7 +623,7 @@ __global__ void __launch_bounds__(SPEC_NT, 4) k_spec_x(Dev d, Fields<float> F, S
 
 // y transforms of column groups of one packed plane, in place on the
 // spectra; the tile keeps the plane's row-major layout (sequences interleaved).
-template <bool MIXED> __global__ void __launch_bounds__(SPEC_NT, 4) k_spec_y(Dev d, SpecDev sp)
+template <int LEN> __global__ void __launch_bounds__(SPEC_NT, 4) k_spec_y(Dev d, SpecDev sp)
 {
     extern __shared__ float2 sm2[];
     const int f = __ldg(sp.by_film + blockIdx.x);
@@ -586,13 +635,14 @@ template <bool MIXED> __global__ void __launch_bounds__(SPEC_NT, 4) k_spec_y(Dev
     const int kk = lb / groups, x0 = (lb - kk * groups) * cb, nc = min(cb, nx - x0);
     const SpecAxis &ay = P.ay;
     float2 *base = sp.C + P.coff + (long long)kk * nx * ny + x0;
-    float2 *a = sm2, *b = sm2 + cb * ny, *tw = sm2 + 2 * cb * ny;
-    for (int t = threadIdx.x; t < ny; t += blockDim.x) tw[t] = __ldg(sp.tw + P.twy + t);
+    const int len = LEN == FFT_CHIRP ? fft_len(ay) : ny;
+    float2 *a = sm2, *b = sm2 + cb * len, *tw = sm2 + 2 * cb * len;
+    fft_twiddles<LEN>(tw, ay, P.twy, sp.tw);
     // sequence c = column x0 + c, element e = row y (coalesced along x)
     auto ld = [&](int c, int e) { return base[(long long)e * nx + c]; };
     auto st = [&](int c, int e, float2 v) { base[(long long)e * nx + c] = v; };
     __syncthreads();                                                     // twiddles
-    fft_any<true, MIXED>(a, b, nc, ay, nc, 1, tw, ld, st);
+    fft_any<true, LEN>(a, b, nc, ay, nc, 1, tw, sp.tw, ld, st);
 }
 
 // In-plane modes m whose mirror -m has an index >= m's, one per z solve:
@@ -728,7 +778,7 @@ __host__ __device__ inline size_t spec_yzy_bytes(int ny, int Mp, int M)
 
 constexpr int SPEC_YZY_NT = 512;
 
-template <bool MIXED> __global__ void __launch_bounds__(SPEC_YZY_NT, 1) k_spec_yzy(Dev d, SpecDev sp)
+template <int LEN> __global__ void __launch_bounds__(SPEC_YZY_NT, 1) k_spec_yzy(Dev d, SpecDev sp)
 {
     extern __shared__ float2 sm2[];
     const int f = __ldg(sp.bq_film + blockIdx.x);
@@ -757,11 +807,11 @@ template <bool MIXED> __global__ void __launch_bounds__(SPEC_YZY_NT, 1) k_spec_y
     for (int t = threadIdx.x; t < ny; t += blockDim.x) tw[t] = __ldg(sp.tw + P.twy + t);
     __syncthreads();
     // forward y transforms: spectra -> tile R
-    float2 *R = (fft_passes<MIXED>(ay) & 1) == 0 ? A : B;
+    float2 *R = (fft_passes<LEN>(ay) & 1) == 0 ? A : B;
     {
         auto ld = [&](int sq, int e) { return gcol(sq)[e]; };
         auto st = [&](int sq, int e, float2 v) { R[spec_pad(sq * ny + e)] = v; };
-        fft_any<false, MIXED>(A, B, nseq, ay, 1, ny, tw, ld, st);
+        fft_any<false, LEN>(A, B, nseq, ay, 1, ny, tw, sp.tw, ld, st);
     }
     cp_wait<0>();
     __syncthreads();
@@ -823,7 +873,7 @@ template <bool MIXED> __global__ void __launch_bounds__(SPEC_YZY_NT, 1) k_spec_y
     // y transforms of the conjugated solutions: tile R -> spectra
     auto ld = [&](int sq, int e) { return R[spec_pad(sq * ny + e)]; };
     auto st = [&](int sq, int e, float2 v) { gcol(sq)[e] = v; };
-    fft_any<false, MIXED>(R, R == A ? B : A, nseq, ay, 1, ny, tw, ld, st);
+    fft_any<false, LEN>(R, R == A ? B : A, nseq, ay, 1, ny, tw, sp.tw, ld, st);
 }
 
 // ------------------------------------------------- Neumann z boundary

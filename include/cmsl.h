@@ -95,8 +95,9 @@ typedef struct {
  * depolarisation solves have the Dirichlet z boundary and nx, ny of the form
  * 2^a 3^b (<= 4096): an in-plane FFT, a tridiagonal solve along z per mode and
  * the inverse FFT.  CMSL_INNER_AUTO also takes it for the Neumann z boundary
- * (mirrored end rows and the pinned cell solved exactly; CMSL_INNER_DIRECT
- * still asks for the Dirichlet boundary).  With one permittivity for all materials it is exact for
+ * (mirrored end rows and the pinned cell solved exactly) and for other sides
+ * up to 2048 (chirp transforms) where every such film has nx ny >= 1024;
+ * CMSL_INNER_DIRECT still asks for the Dirichlet boundary and 2^a 3^b.  With one permittivity for all materials it is exact for
  * the operator up to FP32 rounding.  With several it solves with one
  * reference permittivity (the middle of the range the film's grains use) and
  * preconditions the double-float refinement, whose residual applies the true
