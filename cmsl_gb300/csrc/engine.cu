@@ -1421,22 +1421,6 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
         if (n > cg_per * cg_nsm) e->persistent = false;
     }
 
-    // FP64 PCG: one cooperative launch for every film, resident where every
-    // film's vectors fit the registers of its share of one block per SM
-    int p64_nsm = 0, p64_per = 0;
-    e->pcg64 = e->precision == CMSL_FP64 && e->any_dep && n <= CG_MAX_FILMS && !(tk && atoi(tk) != 0);
-    if (e->pcg64) {
-        int dev = 0, per1 = 0;
-        CK(cudaGetDevice(&dev));
-        CK(cudaDeviceGetAttribute(&p64_nsm, cudaDevAttrMultiProcessorCount, dev));
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&p64_per, k_pcg64, P64_NT, 0));
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per1, k_pcg64r, P64_NT, 0));
-        if (p64_per < 1 || per1 < 1) return fail(CMSL_ERR_CUDA, "FP64 PCG kernel cannot be resident");
-        p64_per = std::min(p64_per, P64_BPS);
-        p64_nsm = std::min(p64_nsm, P64_MAX_BLOCKS / P64_BPS);
-        if (n > p64_nsm) e->pcg64 = false;
-    }
-
     // grain ids are checked on the host (before any device work); the
     // per-cell codes, interface flags and material voxel counts are built on
     // the device below (build_film_codes); work items, film tables
@@ -1471,6 +1455,22 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
         fd.off = h.off;
         fd.g_off = g_off;
         g_off += h.ng;
+    }
+
+    // FP64 PCG: one cooperative launch for every film, resident where every
+    // film's vectors fit the registers of its share of one block per SM
+    int p64_nsm = 0, p64_per = 0;
+    e->pcg64 = e->precision == CMSL_FP64 && e->any_dep && n <= CG_MAX_FILMS && !(tk && atoi(tk) != 0);
+    if (e->pcg64) {
+        int dev = 0, per1 = 0;
+        CK(cudaGetDevice(&dev));
+        CK(cudaDeviceGetAttribute(&p64_nsm, cudaDevAttrMultiProcessorCount, dev));
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&p64_per, k_pcg64, P64_NT, 0));
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per1, k_pcg64r, P64_NT, 0));
+        if (p64_per < 1 || per1 < 1) return fail(CMSL_ERR_CUDA, "FP64 PCG kernel cannot be resident");
+        p64_per = std::min(p64_per, P64_BPS);
+        p64_nsm = std::min(p64_nsm, P64_MAX_BLOCKS / P64_BPS);
+        if (n > p64_nsm) e->pcg64 = false;
     }
 
     // persistent PCG partition: stencil bricks of PZ planes film by film;
