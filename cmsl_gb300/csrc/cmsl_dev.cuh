@@ -89,7 +89,7 @@ struct FilmDev {
                                 // later refinement pass may update r instead of recomputing it
     int direct;                 // FP32_REFINED inner solve by the direct spectral solve
     int defer_ok;               // the check after a step's one direct solve may run inside the next
-                                // TDGL step (upd_ok, warm start at most quadratic)
+                                // TDGL step (upd_ok, one eps, warm start at most quadratic)
     double n_mat[3];            // voxels per material (sum of the reference's masks)
     double rowc[11];            // sweep row: factors of the sums, constants (evolve.cu:391-400)
     Coef<double> coef[6];       // index mat*2 + iface

@@ -1437,12 +1437,12 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
         }
         FilmDev &fd = fds[fi];
         fill_film(fd, dsc, e->precision);
-        // the FP32 update pass r <- r - A dx follows an exact (one-eps) direct solve only;
-        // its check may run inside the next TDGL step when that step's warm start
-        // leaves the third-oldest potential unread
+        // the FP32 update pass r <- r - A dx follows a direct solve; after an
+        // exact one (one eps) its check may run inside the next TDGL step when
+        // that step's warm start leaves the third-oldest potential unread
         fd.direct = e->spectral ? 1 : 0;
-        fd.upd_ok = e->spectral && fd.uni_eps ? 1 : 0;
-        fd.defer_ok = fd.upd_ok && fd.dep_flag && fd.warm <= 2 ? 1 : 0;
+        fd.upd_ok = e->spectral ? 1 : 0;
+        fd.defer_ok = fd.upd_ok && fd.uni_eps && fd.dep_flag && fd.warm <= 2 ? 1 : 0;
         fd.cheb_delta = 0.f;
         if (e->spectral && !fd.uni_eps && fd.dep_flag) {
             double kappa = 1.0;

@@ -908,11 +908,13 @@ __device__ __forceinline__ void refine_film(const Dev &d, int fi, FilmTail &T)
         S->bb = bb;
         const bool fin = fin64(rr);
         const bool conv = fin && (rr <= tol2 * bb || rr == 0.0);
-        // the next pass may update r when this one formed it in full and
-        // ||r|| <= 1e-4 ||b||: the FP32 rounding of A dx (relative ~1e-7,
-        // times the stencil's cancellation) then stays far below the
-        // refinement target; never two update passes in a row
-        const int upd = !was_upd && upd_ok && rr <= 1e-8 * bb;
+        // the next pass may update r when ||r|| <= 1e-4 ||b||: the FP32
+        // rounding of A dx (relative ~1e-7, times the stencil's cancellation)
+        // then stays far below the refinement target.  One eps: when this pass
+        // formed r in full (a second update would hint at a solve gone wrong).
+        // Several: in a row, as the passes of a Chebyshev sequence shrink r by
+        // a factor each, and with it what an update rounds off.
+        const int upd = upd_ok && rr <= 1e-8 * bb && (!was_upd || dl > 0.f);
         S->upd = upd;
         // the next direct solve's increment (Chebyshev semi-iteration for a
         // direct solve preconditioning several eps, M^-1 A's spectrum in

@@ -651,7 +651,10 @@ static __global__ void __launch_bounds__(NT) k_extrap(Dev d)
 // Laplacian (one double-float product per cell, no material codes).
 // An update pass (after the direct solve, once ||r|| <= 1e-4 ||b||) instead
 // forms r <- r - A dx in FP32: dx is then small, and the FP32 rounding of
-// A dx stays far below the refinement target.
+// A dx stays far below the refinement target.  With several eps, whose steps
+// take five to eight passes, it reads dx and the codes where the full pass
+// reads the potential, P and D^-1 with halos and works in double-float: 53.4
+// -> 24.7 us a pass at 256x256x32, the step 692 -> 499 us.
 // No FP64 instruction is executed.
 constexpr int R32_NS = 5;
 
@@ -724,7 +727,7 @@ __device__ __forceinline__ void refine_cell(const RConst &rc, int k, bool ident,
     } else {
         if (upd) rv = r_old + minus_adx<UNI>(rc, k, c);
         else refine_row<UNI>(rc, k, c, rv, bh);
-        wj = UNI ? rc.dinv_u : dinv;
+        wj = UNI ? rc.dinv_u : upd ? 1.f : dinv;    // several eps: only the sign of the update's third sum is used
     }
     acc[0] = fmaf(rv, rv, acc[0]);
     acc[1] = fmaf(bh, bh, acc[1]);
@@ -773,7 +776,7 @@ __global__ void __launch_bounds__(TileShape<TYc>::NTt, TileShape<TYc>::MINB) k_r
     rc.cf_l = f->cf_l;
     const bool run_ = f->dep_flag != 0 && (d.force || S->outer_active);
     const bool apply_ = S->refine > 0;                  // later pass: x = phi + dx; first: the warm start
-    const bool upd_ = UNI && apply_ && S->upd && f->upd_ok;   // r <- r - A dx (after the direct solve, one eps)
+    const bool upd_ = apply_ && S->upd && f->upd_ok;     // r <- r - A dx (after the direct solve)
     const int cur = d.ctl->cur, fr = phi_free(S);
     const long long off = f->off, fs = d.ncells;
     const float2 *xh = phi2_sel(d, apply_ ? S->phi_cur : fr) + off;
@@ -792,13 +795,17 @@ __global__ void __launch_bounds__(TileShape<TYc>::NTt, TileShape<TYc>::MINB) k_r
         if (run && p <= zhi) {
             const int so = g.own_slot, sh = g.halo_slot;
             if (upd) {
-                // update pass: dx with its halo; phi and the old r of the own cell
+                // update pass: dx (several eps: and the codes) with its halo; phi and the old r of the own cell
                 if (g.valid) {
                     cp8(st + L::FX + 2 * so, xh + own_o);
                     cp4(st + L::DX + so, dx + own_o);
                     cp4(st + L::PZ + threadIdx.x, r + own_o);
+                    if (!UNI) cp4(st + L::CODE + so, code + own_o);
                 }
-                if (g.halo) cp4(st + L::DX + sh, dx + halo_o);
+                if (g.halo) {
+                    cp4(st + L::DX + sh, dx + halo_o);
+                    if (!UNI) cp4(st + L::CODE + sh, code + halo_o);
+                }
             } else {
                 if (g.valid) {
                     cp8(st + L::FX + 2 * so, xh + own_o);
@@ -871,14 +878,14 @@ __global__ void __launch_bounds__(TileShape<TYc>::NTt, TileShape<TYc>::MINB) k_r
             // identity rows: the Dirichlet planes, or the Neumann pin
             const bool ident = rq.neu ? k == kpin : (k == 0 || k == nz - 1);
             float rv;
-            refine_cell<UNI>(rq, k, ident, upd, c, upd ? sk[L::PZ + tz] : 0.f, UNI ? 0.f : sk[L::DINV + tz], rv, acc);
+            refine_cell<UNI>(rq, k, ident, upd, c, upd ? sk[L::PZ + tz] : 0.f, UNI || upd ? 0.f : sk[L::DINV + tz], rv, acc);
             r[o] = rv;
             if (apply) nh[o] = make_float2(c.xc.h, c.xc.l);
         }
     };
     if (!run_ || rc.neu) planes(Mode<0>{});
     else if (!apply_) planes(Mode<1>{});
-    else if (UNI && upd_) planes(Mode<UNI ? 3 : 2>{});
+    else if (upd_) planes(Mode<3>{});
     else planes(Mode<2>{});
     cp_wait<0>();
     if (run_) block_total32<3>(d, it.x, 1, acc, sRed);
