@@ -1910,9 +1910,9 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
         // last block
         const bool fb = n > 1;
         if (fb) {
-            e->refine_cp[0] = uni ? (void *)k_refine32<true, R32_NS, 4, true> : (void *)k_refine32<false, R32_NS, 4, true>;
-            e->refine_cp[1] = uni ? (void *)k_refine32<true, R32_NS, 8, true> : (void *)k_refine32<false, R32_NS, 8, true>;
-            e->refine_cp[2] = uni ? (void *)k_refine32<true, R32_NS, 16, true> : (void *)k_refine32<false, R32_NS, 16, true>;
+            e->refine_cp[0] = uni ? (void *)k_refine32<true, r32_ns<true>(), 4, true> : (void *)k_refine32<false, r32_ns<false>(), 4, true>;
+            e->refine_cp[1] = uni ? (void *)k_refine32<true, r32_ns<true>(), 8, true> : (void *)k_refine32<false, r32_ns<false>(), 8, true>;
+            e->refine_cp[2] = uni ? (void *)k_refine32<true, r32_ns<true>(), 16, true> : (void *)k_refine32<false, r32_ns<false>(), 16, true>;
             e->tdgl_cp[0] = (void *)k_tdgl32<T32_NS, 4, false, true>;
             e->tdgl_cp[1] = (void *)k_tdgl32<T32_NS, 8, false, true>;
             e->tdgl_cp[2] = (void *)k_tdgl32<T32_NS, 16, false, true>;
@@ -1920,9 +1920,9 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
             e->tdgl_def[1] = (void *)k_tdgl32<T32_NS, 8, true, true>;
             e->tdgl_def[2] = (void *)k_tdgl32<T32_NS, 16, true, true>;
         } else {
-            e->refine_cp[0] = uni ? (void *)k_refine32<true, R32_NS, 4> : (void *)k_refine32<false, R32_NS, 4>;
-            e->refine_cp[1] = uni ? (void *)k_refine32<true, R32_NS, 8> : (void *)k_refine32<false, R32_NS, 8>;
-            e->refine_cp[2] = uni ? (void *)k_refine32<true, R32_NS, 16> : (void *)k_refine32<false, R32_NS, 16>;
+            e->refine_cp[0] = uni ? (void *)k_refine32<true, r32_ns<true>(), 4> : (void *)k_refine32<false, r32_ns<false>(), 4>;
+            e->refine_cp[1] = uni ? (void *)k_refine32<true, r32_ns<true>(), 8> : (void *)k_refine32<false, r32_ns<false>(), 8>;
+            e->refine_cp[2] = uni ? (void *)k_refine32<true, r32_ns<true>(), 16> : (void *)k_refine32<false, r32_ns<false>(), 16>;
             e->tdgl_cp[0] = (void *)k_tdgl32<T32_NS, 4>;
             e->tdgl_cp[1] = (void *)k_tdgl32<T32_NS, 8>;
             e->tdgl_cp[2] = (void *)k_tdgl32<T32_NS, 16>;

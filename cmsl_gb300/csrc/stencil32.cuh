@@ -656,7 +656,11 @@ static __global__ void __launch_bounds__(NT) k_extrap(Dev d)
 // reads the potential, P and D^-1 with halos and works in double-float: 53.4
 // -> 24.7 us a pass at 256x256x32, the step 692 -> 499 us.
 // No FP64 instruction is executed.
-constexpr int R32_NS = 5;
+// Stages of the ring.  Several eps: four, since the codes and D^-1 make a stage
+// 10 KB and four blocks' five stages leave the L1 28 KB (256x256x32 with
+// 50 / 30 / 15: a step 498 -> 489 us); one eps: five of 8 KB (four: 512x512x64
+// first pass 128 -> 142 us).
+template <bool UNI> constexpr int r32_ns() { return UNI ? 5 : 4; }
 
 // sum of six double-float values minus 6 c; the hi parts are summed error-free
 __device__ __forceinline__ df lap7(df e, df w, df n, df s, df u, df dn, df c)
@@ -745,7 +749,7 @@ template <bool UNI, int TYc = TY> struct R32Lay {
 };
 template <bool UNI, int TYc = TY> constexpr size_t r32_smem()
 {
-    return sizeof(float) * R32_NS * R32Lay<UNI, TYc>::STAGE;
+    return sizeof(float) * r32_ns<UNI>() * R32Lay<UNI, TYc>::STAGE;
 }
 
 template <bool UNI, int NS, int TYc = TY, bool FB = false>
