@@ -1696,6 +1696,13 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
         long long coff = 0;
         size_t smx = 0, smy = 0;
         bool chirp = false;                                         // a chirp transform among the films
+        long long lines_x = 0, lines_y = 0;                         // rows and columns of the films' packed planes
+        for (const FilmHost &h : e->fh)
+            if (h.dep) {
+                const long long mp = (h.nz - (h.zbc == CMSL_DIRICHLET ? 2 : 0) + 1) / 2;
+                lines_x += mp * h.ny;
+                lines_y += mp * h.nx;
+            }
         auto tables = [&](int nn, int *two, int *lamo) {
             *two = (int)tw.size();
             *lamo = (int)lam.size();
@@ -1741,9 +1748,11 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
                 }
             chirp |= P.ax.lgm || P.ay.lgm;
             // rows (columns) per transform block: about two blocks per SM for
-            // the film's Mp ny rows (Mp nx columns), a power of two, at most
+            // all films' rows (columns) together, a power of two, at most
             // SPEC_ELEMS values (8 rows of 256 at 256x256x32, 8 of 512 at
-            // 512x512x64, 1 of 64 at 64x64x16); CMSL_SPEC_RB fixes it
+            // 512x512x64, 1 of 64 at 64x64x16); CMSL_SPEC_RB fixes it.  (By
+            // every film's own rows, a batch of 16 films took blocks of 1 to 8
+            // rows whose threads mostly idled: a solve 219 us, now 141.)
             const char *rbe = getenv("CMSL_SPEC_RB");
             auto per_block = [&](long long lines, int len) {
                 const int cap = std::max(1, SPEC_ELEMS / len);
@@ -1752,8 +1761,7 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
                 if (rbe && atoi(rbe) > 0) r = std::min(cap, atoi(rbe));
                 return r;
             };
-            const int rbx = per_block((long long)P.Mp * h.ny, fft_len(P.ax)),
-                      cby = per_block((long long)P.Mp * h.nx, fft_len(P.ay));
+            const int rbx = per_block(lines_x, fft_len(P.ax)), cby = per_block(lines_y, fft_len(P.ay));
             P.rb = rbx;
             P.cb = cby;
             const long long gx = ((long long)P.Mp * h.ny + rbx - 1) / rbx;
