@@ -349,6 +349,7 @@ extern "C" cmsl_status cmsl_film_loop_gradient(cmsl_film *f, int n_steps, const 
         TRY(forward_segment(e, st, Ez + s0, row + s0, len, j == nseg - 1 ? store : nullptr, cur));
         CK(cudaStreamSynchronize(st));
     }
+    TRY(check_waits(e));
     {
         SolveDev S;
         CK(cudaMemcpy(&S, e->d_solve, sizeof(SolveDev), cudaMemcpyDeviceToHost));
@@ -432,6 +433,7 @@ extern "C" cmsl_status cmsl_film_loop_gradient(cmsl_film *f, int n_steps, const 
         CK(cudaStreamSynchronize(st));
     }
 
+    TRY(check_waits(e));
     // ---- theta partials -> d loss / d (alpha, beta, gamma, g, kappa) per material
     std::vector<double> th((size_t)NTH * nit);
     CK(cudaMemcpy(th.data(), tacc, sizeof(double) * th.size(), cudaMemcpyDeviceToHost));

@@ -101,11 +101,13 @@ struct FilmDev {
     float cb_h, cb_l;           // eps_0_nd / (2 h) as a double-float pair
 };
 
+constexpr int SOLVE_WAIT = 4;       // SolveDev::status: a bounded wait of the solve gave up
+
 struct SolveDev {               // per film, lives in device memory
     double rz, rz0, pq, alpha, beta, rr, bb, rr64;
     int iters;                  // PCG iterations of the current (inner) solve
     int active;                 // inner PCG still running
-    int status;                 // 0 ok, 1 breakdown, 2 bad initial residual, 3 refine cap
+    int status;                 // 0 ok, 1 breakdown, 2 bad initial residual, 3 refine cap, SOLVE_WAIT
     int outer_active;           // FP32_REFINED: refinement still running
     int refine;                 // refinement passes this step
     int total_iters;            // PCG iterations this step

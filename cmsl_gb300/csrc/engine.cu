@@ -884,6 +884,24 @@ inline double *locked_dst(double *p)
     return a.type == cudaMemoryTypeHost ? (double *)a.devicePointer : nullptr;
 }
 
+// Bounded waits that gave up since the last look (the persistent PCGs'
+// exchanges, the tensor copies), reported once: what they left is no result.
+cmsl_status check_waits(Engine *e)
+{
+    int pcg = 0, copy = 0;
+    if (e->cg.err) CK(cudaMemcpy(&pcg, e->cg.err, sizeof(int), cudaMemcpyDeviceToHost));
+    if (e->d_err) CK(cudaMemcpy(&copy, e->d_err, sizeof(int), cudaMemcpyDeviceToHost));
+    if (pcg) {
+        CK(cudaMemset(e->cg.err, 0, sizeof(int)));
+        return fail(CMSL_ERR_CUDA, "persistent PCG grid barrier timed out");
+    }
+    if (copy & TMA_ERR_WAIT) {
+        CK(cudaMemset(e->d_err, 0, sizeof(int)));
+        return fail(CMSL_ERR_CUDA, "a tensor-copy wait of a stencil pass timed out");
+    }
+    return CMSL_OK;
+}
+
 }  // namespace cmsl_eng
 
 namespace {
@@ -2186,16 +2204,7 @@ cmsl_status sync(Engine *e, int32_t *film_status)
     CK(cudaGetLastError());
     std::vector<SolveDev> S((size_t)e->n_films);
     CK(cudaMemcpy(S.data(), e->d_solve, sizeof(SolveDev) * S.size(), cudaMemcpyDeviceToHost));
-    if (e->cg.err) {
-        int err = 0;
-        CK(cudaMemcpy(&err, e->cg.err, sizeof(int), cudaMemcpyDeviceToHost));
-        if (err) return fail(CMSL_ERR_CUDA, "persistent PCG grid barrier timed out");
-    }
-    if (e->d_err) {
-        int err = 0;
-        CK(cudaMemcpy(&err, e->d_err, sizeof(int), cudaMemcpyDeviceToHost));
-        if (err & TMA_ERR_WAIT) return fail(CMSL_ERR_CUDA, "a tensor-copy wait of a stencil pass timed out");
-    }
+    TRY(check_waits(e));
     int first = -1;
     for (int fi = 0; fi < e->n_films; ++fi) {
         if (film_status) film_status[fi] = S[fi].sticky;
@@ -2203,6 +2212,7 @@ cmsl_status sync(Engine *e, int32_t *film_status)
     }
     if (first >= 0) {
         const int s = S[first].sticky;
+        if (s == SOLVE_WAIT) return fail(CMSL_ERR_CUDA, "persistent PCG grid barrier timed out");
         const char *what = s == 1 ? "breakdown" : "invalid initial residual";
         if (e->n_films > 1)
             return fail(CMSL_ERR_PCG, "PCG failure (status %d: %s) in at least one step of film %d", s, what, first);
@@ -2669,7 +2679,8 @@ cmsl_status cmsl_film_depol(cmsl_film *f, int32_t *iters, int32_t *status)
     CK(cudaMemcpy(&S, f->d_solve, sizeof(SolveDev), cudaMemcpyDeviceToHost));
     if (iters) { iters[0] = S.total_iters; if (f->precision != CMSL_FP64) iters[1] = S.refine; }
     if (status) *status = S.status;
-    return CMSL_OK;
+    // FP64 slots carry a wait that gave up; the FP32 PCG's are in its error word only
+    return S.status == SOLVE_WAIT || f->persistent ? check_waits(f) : CMSL_OK;
 }
 
 // Depol_field over caller device arrays: Pm in, phi (warm start in,
@@ -2746,7 +2757,7 @@ cmsl_status cmsl_film_depol_device(cmsl_film *f, const double *Pmx, const double
     CK(cudaStreamSynchronize(st));
     if (iters) { iters[0] = S.total_iters; iters[1] = f->precision != CMSL_FP64 ? S.refine : 0; }
     if (status) *status = S.status;
-    return CMSL_OK;
+    return S.status == SOLVE_WAIT || f->persistent ? check_waits(f) : CMSL_OK;
 }
 
 cmsl_status cmsl_film_apply_operator(cmsl_film *f, const double *x, double *y)

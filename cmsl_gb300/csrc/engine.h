@@ -234,6 +234,7 @@ cmsl_status add_while(cudaGraph_t g, cudaGraphNode_t *node, const cudaGraphNode_
                       cudaGraphConditionalHandle h, cudaGraph_t *body);
 cmsl_status add_pcg64(cudaGraph_t g, cudaGraphNode_t *node, const cudaGraphNode_t *dep, const Engine *e, Dev d);
 cmsl_status build_graph(Engine *e);
+cmsl_status check_waits(Engine *e);
 
 }  // namespace cmsl_eng
 

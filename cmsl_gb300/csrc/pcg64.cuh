@@ -37,7 +37,10 @@
 // are 61 us).
 //
 // Waits are bounded (Pcg64::spin_limit); a wait that gives up records an error
-// and its block leaves.
+// and its block leaves.  Where the film's first block leaves so, the solve's
+// status is SOLVE_WAIT; where only others do, they gave up on sums that the
+// first block still received, and the solve it reports is complete or ends on
+// a wait of its own for theirs.
 #pragma once
 #include "kernels.cuh"
 
@@ -336,8 +339,8 @@ __device__ __forceinline__ void p64_done(SolveDev *S, const P64Scal &s, int iter
     S->rz = s.rz;
     S->rr = s.rr;
     S->active = 0;
-    if (s.go == -2) {
-        S->status = 1;
+    if (s.go < 0) {
+        S->status = s.go == -2 ? 1 : SOLVE_WAIT;
         S->outer_active = 0;
     }
 }

@@ -166,7 +166,10 @@ cmsl_status cmsl_film_get_iters(cmsl_film *film, int n, int32_t *pcg_iters, int3
  *  - depol: one Depol_field (RHS from the current Pm, warm-started PCG);
  *  - apply_operator: y = A x with the film's operator (apply_A), FP64 or FP32;
  *  - efield: E = -grad(phi) of the current phi (Calc_EfieldMag; FP32-refined
- *    films difference the double-float potential in FP64). */
+ *    films difference the double-float potential in FP64).
+ * depol's status: 0 solved (or the iteration cap), 1 breakdown, 2 invalid
+ * initial residual, 3 refinement cap, 4 a bounded wait of the solver gave up
+ * (the call then returns CMSL_ERR_CUDA, as cmsl_film_sync after such a run). */
 cmsl_status cmsl_film_tdgl_step(cmsl_film *film, double Ez);
 cmsl_status cmsl_film_depol(cmsl_film *film, int32_t *iters, int32_t *status);
 cmsl_status cmsl_film_apply_operator(cmsl_film *film, const double *x, double *y);
@@ -181,7 +184,7 @@ cmsl_status cmsl_film_diag_inv(cmsl_film *film, double *dinv);
  * so a caller keeps one film for its grid and calls this once per step.  The
  * film's own P state is overwritten (its Pm with the given one).  Single
  * films with a depolarisation solve; iters[0] PCG iterations, iters[1]
- * refinement passes (FP32_REFINED). */
+ * refinement passes (FP32_REFINED); status as cmsl_film_depol's. */
 cmsl_status cmsl_film_depol_device(cmsl_film *film, const double *Pmx, const double *Pmy, const double *Pmz,
                                    double *phi, double *Ex, double *Ey, double *Ez, void *stream,
                                    int32_t *iters, int32_t *status);

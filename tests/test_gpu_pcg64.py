@@ -114,3 +114,36 @@ def test_pcg64_wait_timeout_is_reported(gpu):
         h.set_state(P)
         h.run(np.full(2, 0.1))
         assert all(np.isfinite(p).all() for p in h.get_state()[0])
+
+
+@pytest.mark.parametrize("form", ["resident", "streaming"])
+def test_pcg64_wait_timeout_ends_single_calls(gpu, form, monkeypatch):
+    """The calls that solve without a run -- depol, depol on device arrays, the
+    loop gradient -- end on such a wait with CMSL_ERR_CUDA too, not with an
+    unfinished potential; the wait is reported once."""
+    import ctypes as C
+
+    import torch
+    from cmsl_gb300._lib import lib
+    f, P = random_film(64, 32, 8, seed=71, eps_0_nd=3.0, p_scale=0.2)
+    monkeypatch.setenv("CMSL_P64_STREAM", "1" if form == "streaming" else "0")
+    monkeypatch.setenv("CMSL_PCG_HOLD_BLOCK", "1")
+    monkeypatch.setenv("CMSL_PCG_SPIN_LIMIT", "2000")
+    with gpu.Film.from_oracle_film(f) as g:
+        g.set_state(P)
+        with pytest.raises(gpu.CmslError) as e:
+            g.depol()
+        assert e.value.status == 2 and "barrier timed out" in str(e.value)
+        assert lib().cmsl_film_sync(g._h) == 0
+
+        t = [torch.from_numpy(p).cuda() for p in P[:3]] + [torch.zeros(f.N, dtype=torch.float64, device="cuda") for _ in range(4)]
+        it, st = np.zeros(2, np.int32), np.zeros(1, np.int32)
+        ip = C.POINTER(C.c_int32)
+        assert lib().cmsl_film_depol_device(g._h, *[C.c_void_p(v.data_ptr()) for v in t], None, it.ctypes.data_as(ip),
+                                            st.ctypes.data_as(ip)) == 2
+        assert st[0] == 4
+
+        g.set_state(P)
+        with pytest.raises(gpu.CmslError) as e:
+            g.loop_gradient(np.full(2, 0.1), np.arange(2, dtype=np.int32), np.zeros(2), 2)
+        assert e.value.status == 2 and "barrier timed out" in str(e.value)
