@@ -87,6 +87,9 @@ struct FilmDev {
                                 // the half-width of M^-1 A's spectrum around 1 (0: exact solve)
     int upd_ok;                 // FP32_REFINED: the inner solve leaves r intact (direct solve), so a
                                 // later refinement pass may update r instead of recomputing it
+    float upd_c;                // what an update pass rounds off, relative to ||A dx|| (0: one eps, whose single
+                                // update per step stays below every target the FP32 solve reaches)
+    float refine_tolf;          // sqrt(refine_tol2)
     int direct;                 // FP32_REFINED inner solve by the direct spectral solve
     int defer_ok;               // the check after a step's one direct solve may run inside the next
                                 // TDGL step (upd_ok, one eps, warm start at most quadratic)
@@ -123,6 +126,7 @@ struct SolveDev {               // per film, lives in device memory
     int inner_max;              // inner iteration cap of the current pass
     int upd;                    // the next refinement pass updates r <- r - A dx (FP32) instead of
                                 // forming b - A phi in double-float
+    float upd_err;              // what the updates up to the next pass may have rounded off r, over ||b||
     float cheb_rho;             // Chebyshev recurrence of the preconditioned refinement (rho_k)
     float cheb_w, cheb_m;       // the next direct solve's increment: dx <- w M^-1 r + m dx
     float pin_r, pin_x;         // direct solve of a Neumann film: r and the previous increment at the pinned cell

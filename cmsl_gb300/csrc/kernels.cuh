@@ -345,6 +345,17 @@ __device__ __forceinline__ void film_tail(const Dev &d, int fi, int kind, FilmTa
     __syncthreads();
 }
 
+// sqrt(a / b) of two squared norms as a float (values below 1e-19 count as 0),
+// without the FP64 pipe: both scaled by b's exponent.
+__device__ __forceinline__ float rel_norm(double a, double b)
+{
+    const int ea = (__double2hiint(a) >> 20) & 0x7ff, eb = (__double2hiint(b) >> 20) & 0x7ff;
+    if (ea == 0 || ea - eb <= -126) return 0.f;
+    if (eb == 0 || ea - eb >= 127) return __int_as_float(0x7f800000);
+    auto at = [](double v, int e) { return (float)__hiloint2double((__double2hiint(v) & 0xfffff) | (e << 20), __double2loint(v)); };
+    return sqrtf(at(a, 1023 + ea - eb) / at(b, 1023));
+}
+
 // A double is finite / positive, without the FP64 pipe.
 __device__ __forceinline__ bool fin64(double v) { return ((unsigned)__double2hiint(v) & 0x7ff00000u) != 0x7ff00000u; }
 
@@ -883,7 +894,7 @@ __device__ __forceinline__ void refine_film(const Dev &d, int fi, FilmTail &T)
     const double tol2 = ff->refine_tol2;
     const int dep = ff->dep_flag, upd_ok = ff->upd_ok, defer_ok = ff->defer_ok, max_refine = ff->max_refine;
     const int direct = ff->direct, inner_max = ff->inner_max;
-    const float dl = ff->cheb_delta;
+    const float dl = ff->cheb_delta, uc = ff->upd_c, tol = ff->refine_tolf;
     if (!dep) return;
     film_tail<3>(d, fi, 1, T);
     if (threadIdx.x == 0 && !d.force && T.S.outer_active) {       // kernel timing: the state stays as it is
@@ -907,15 +918,25 @@ __device__ __forceinline__ void refine_film(const Dev &d, int fi, FilmTail &T)
         S->rr64 = rr;
         S->bb = bb;
         const bool fin = fin64(rr);
-        const bool conv = fin && (rr <= tol2 * bb || rr == 0.0);
+        // what the updates since the last full pass may have rounded off, which
+        // later ones do not bring back into r: uc (FilmDev::upd_c) of
+        // ||A dx|| <= ||r before|| + ||r after|| each, all over ||b||
+        const float q = uc > 0.f ? rel_norm(rr, bb) : 0.f;
+        const float lost = was_upd ? P.upd_err + uc * q : 0.f;
+        const bool conv = fin && (rr <= tol2 * bb || rr == 0.0) && (lost == 0.f || q + lost <= tol);
         // the next pass may update r when ||r|| <= 1e-4 ||b||: the FP32
         // rounding of A dx (relative ~1e-7, times the stencil's cancellation)
         // then stays far below the refinement target.  One eps: when this pass
         // formed r in full (a second update would hint at a solve gone wrong).
         // Several: in a row, as the passes of a Chebyshev sequence shrink r by
-        // a factor each, and with it what an update rounds off.
-        const int upd = upd_ok && rr <= 1e-8 * bb && (!was_upd || dl > 0.f);
+        // a factor each, and with it what an update rounds off -- while that
+        // stays within a quarter of the target (at refine_tol 1e-8 it does from
+        // the first 1e-4 on; at 1e-11 updates that ran from 1e-4 left 1.4 times
+        // the target in b - A phi, at 1e-12 five to eleven times)
+        const float lose = lost + uc * q;
+        const int upd = upd_ok && rr <= 1e-8 * bb && (!was_upd || dl > 0.f) && lose <= 0.25f * tol;
         S->upd = upd;
+        S->upd_err = lose;
         // the next direct solve's increment (Chebyshev semi-iteration for a
         // direct solve preconditioning several eps, M^-1 A's spectrum in
         // [1 - delta, 1 + delta]): solve 0 of a step dx = M^-1 r, then
