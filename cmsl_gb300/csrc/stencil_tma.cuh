@@ -300,7 +300,7 @@ __global__ void __launch_bounds__(NT, 4) k_refine32t(Dev d, Fields<float> F)
     rc.cf_l = f->cf_l;
     const bool run = f->dep_flag != 0 && (d.force || S->outer_active);
     const bool apply = S->refine > 0;                   // later pass: x = phi + dx; first: the warm start
-    const bool upd = UNI && apply && S->upd && f->upd_ok;   // r <- r - A dx (after the direct solve, one eps)
+    const bool upd = apply && S->upd && f->upd_ok;      // r <- r - A dx (after the direct solve)
     const int cur = d.ctl->cur, fr = phi_free(S), xb = apply ? S->phi_cur : fr;
     const long long off = f->off;
     float2 *nh = phi2_sel(d, fr) + off;
@@ -309,10 +309,10 @@ __global__ void __launch_bounds__(NT, 4) k_refine32t(Dev d, Fields<float> F)
     const FilmMaps *M = d.maps + it.x;
 
     auto R = ring_setup<NS, RT_OPS>(smem_rt, bar, ops, zlo, run ? zhi : -1, STAGE);
-    // update pass: dx with its halo, phi and the old r of the own cell;
+    // update pass: dx (several eps: and the codes) with its halo, phi and the old r of the own cell;
     // otherwise x with its halo, dx (later passes), (Pmx, Pmy), Pmz, codes and D^-1
-    R.n_ops = upd ? 7 : 5 + (apply ? 5 : 0) + 5 + 1 + (UNI ? 0 : 6);
-    R.tx = (uint32_t)(upd ? BODY2 + REG1 + BODY1
+    R.n_ops = upd ? (UNI ? 7 : 12) : 5 + (apply ? 5 : 0) + 5 + 1 + (UNI ? 0 : 6);
+    R.tx = (uint32_t)(upd ? BODY2 + REG1 + BODY1 + (UNI ? 0 : REG1)
                           : REG2 + (apply ? REG1 : 0) + REG2 + BODY2 + (UNI ? 0 : REG1 + BODY1));
     if (threadIdx.x == 0) {
         OpBuilder b{ops, 0, x0, y0, nx, ny};
@@ -320,6 +320,7 @@ __global__ void __launch_bounds__(NT, 4) k_refine32t(Dev d, Fields<float> F)
             b.body(phi_maps(M, xb), RT_X, -1, 8);
             b.region(M->x, RT_DX, -1, 4);
             b.add(&M->r, RT_PZ, x0, y0, -1);
+            if (!UNI) b.region(M->code, RT_CODE, -1, 4);
         } else {
             b.region(phi_maps(M, xb), RT_X, -1, 8);
             if (apply) b.region(M->x, RT_DX, -1, 4);
@@ -379,7 +380,7 @@ __global__ void __launch_bounds__(NT, 4) k_refine32t(Dev d, Fields<float> F)
         const bool ident = rc.neu ? (long long)k * plane == pin : (k == 0 || k == nz - 1);
         float rv;
         const float r_old = upd ? ((const float *)(sk + RT_PZ))[tz] : 0.f;
-        refine_cell<UNI>(rc, k, ident, upd, c, r_old, UNI ? 0.f : ((const float *)(sk + RT_DINV))[tz], rv, acc);
+        refine_cell<UNI>(rc, k, ident, upd, c, r_old, UNI || upd ? 0.f : ((const float *)(sk + RT_DINV))[tz], rv, acc);
         r[o] = rv;
         if (apply) nh[o] = make_float2(c.xc.h, c.xc.l);
     }

@@ -105,3 +105,23 @@ def test_update_tight_target(gpu, shape, ratio, zbc, tol):
         pin = f.nx // 2 + f.nx * (f.ny // 2 + (f.nz // 2) * f.ny)
         b[pin], r[pin] = 0.0, 0.0
     assert np.linalg.norm(r) <= 1.05 * tol * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("zbc", [oracle.DIRICHLET, oracle.NEUMANN])
+def test_update_by_tensor_copies(gpu, zbc, monkeypatch):
+    """Residual passes by tensor copies update r where the ring's do: the same
+    arithmetic in the same order, so the same bits and pass counts."""
+    f, P = _film((64, 24, 10), 3.3, 11, zbc)
+    Ez = np.linspace(0.0, 0.3, 6)
+    out = []
+    for staging in ("00", "01"):
+        monkeypatch.setenv("CMSL_STAGING", staging)
+        with gpu.Film.from_oracle_film(f, precision=gpu.FP32_REFINED, refine_tol=1e-8) as g:
+            assert g.tile_config()["residual_staging"] == ("cp.async ring", "tensor copies")[int(staging[1])]
+            g.set_state(P)
+            g.run(Ez)
+            out.append((*g.get_state(), *g.iters()))
+    for a, b in zip(out[0][0], out[1][0]):
+        assert np.array_equal(a, b)
+    for a, b in zip(out[0][1:], out[1][1:]):
+        assert np.array_equal(a, b)
