@@ -87,8 +87,8 @@ struct FilmDev {
                                 // the half-width of M^-1 A's spectrum around 1 (0: exact solve)
     int upd_ok;                 // FP32_REFINED: the inner solve leaves r intact (direct solve), so a
                                 // later refinement pass may update r instead of recomputing it
-    float upd_c;                // what an update pass rounds off, relative to ||A dx|| (0: one eps, whose single
-                                // update per step stays below every target the FP32 solve reaches)
+    float upd_c;                // what an update pass rounds off, relative to ||A dx|| (0: one eps and the
+                                // Dirichlet z boundary, whose one update in a row leaves no more than a full pass)
     float refine_tolf;          // sqrt(refine_tol2)
     int direct;                 // FP32_REFINED inner solve by the direct spectral solve
     int defer_ok;               // the check after a step's one direct solve may run inside the next

@@ -1460,14 +1460,14 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
         // that step's warm start leaves the third-oldest potential unread
         fd.direct = e->spectral ? 1 : 0;
         fd.upd_ok = e->spectral ? 1 : 0;
-        // an update pass with several eps sums six fluxes e_f (dx_f - dx_c): a
-        // few units in the last place (rms 1.6) of fluxes that exceed their sum
-        // by a smooth mode's wavelength over 2 pi: 2 nz with the Dirichlet
-        // planes, the sides with the Neumann ones
+        // an update pass with several eps or the Neumann boundary sums six
+        // fluxes e_f (dx_f - dx_c): a few units in the last place (rms 1.6) of
+        // fluxes that exceed their sum by a smooth mode's wavelength over 2 pi:
+        // 2 nz with the Dirichlet planes, the sides with the Neumann ones
         {
             double len = dsc->nz / M_PI;
             if (dsc->zbc != CMSL_DIRICHLET) len = std::max(len, std::max(dsc->nx, dsc->ny) / (2.0 * M_PI));
-            fd.upd_c = fd.uni_eps ? 0.f : (float)(4.0 * std::ldexp(1.0, -24) * std::max(1.0, len));
+            fd.upd_c = fd.uni_eps && dsc->zbc == CMSL_DIRICHLET ? 0.f : (float)(4.0 * std::ldexp(1.0, -24) * std::max(1.0, len));
             fd.refine_tolf = (float)std::sqrt(fd.refine_tol2);
         }
         fd.defer_ok = fd.upd_ok && fd.uni_eps && fd.dep_flag && fd.warm <= 2 ? 1 : 0;

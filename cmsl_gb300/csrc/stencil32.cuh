@@ -135,7 +135,15 @@ __device__ __forceinline__ float minus_adx(const RConst &rc, int k, const RCell 
 {
     float du, ddn;
     zpick<float>(rc, k, c.du, c.dd, du, ddn);
-    if (UNI) return rc.cu.h * ((c.de + c.dw) + (c.dn + c.ds) + (du + ddn) - 6.f * c.dc);
+    if (UNI) {
+        // Neumann: modes of a whole side, and the constant that meets the pinned
+        // cell, are far larger than their differences; the sum below rounds at
+        // 6 |dx|, 1e-3 of A dx for a mode of 512 cells
+        if (rc.neu)
+            return rc.cu.h * (((c.de - c.dc) + (c.dw - c.dc)) + ((c.dn - c.dc) + (c.ds - c.dc)) +
+                              ((du - c.dc) + (ddn - c.dc)));
+        return rc.cu.h * ((c.de + c.dw) + (c.dn + c.ds) + (du + ddn) - 6.f * c.dc);
+    }
     int mu, md;
     zpick<int>(rc, k, c.mu, c.md, mu, md);
     const float *ch = rc.cf_h + c.mc * 3;
@@ -528,11 +536,22 @@ __device__ __forceinline__ void tdgl_def_film(const Dev &d, int rs, int fi, Film
     __syncthreads();            // T is the next film's
 }
 
-// A pending film's check passed (NaN fails); rr read past this block's L1.
+// A pending film's check passed (NaN fails): the update pass's test, with what
+// the update may have rounded off (refine_film).
+__device__ __forceinline__ bool check_met(const FilmDev *f, double rr, double bb, float upd_err)
+{
+    if (rr == 0.0) return true;
+    if (!(rr <= f->refine_tol2 * bb)) return false;
+    const float uc = f->upd_c;
+    if (uc == 0.f) return true;
+    const float q = rel_norm(rr, bb);
+    return q + (upd_err + uc * q) <= f->refine_tolf;
+}
+// The same of film fi's slot; rr read past this block's L1.
 __device__ __forceinline__ bool def_check_ok(const Dev &d, int fi)
 {
     const double rr = *(volatile const double *)&d.solve[fi].rr64;
-    return rr <= d.films[fi].refine_tol2 * d.solve[fi].bb || rr == 0.0;
+    return check_met(d.films + fi, rr, d.solve[fi].bb, d.solve[fi].upd_err);
 }
 
 // What depends on every film: resolve and begin, or reopen.
@@ -588,8 +607,8 @@ __device__ __forceinline__ void tdgl_def_grid1(const Dev &d, int rs, FilmTail &T
         const FilmDev *f = d.films;
         const double rr = T.tot[7];
         const bool pend = f->dep_flag && T.S.pending;
-        const bool ok = rr <= f->refine_tol2 * T.S.bb || rr == 0.0;
-        if (!pend || ok) {
+        const bool ok = !pend || check_met(f, rr, T.S.bb, T.S.upd_err);
+        if (ok) {
             if (T.S.pending) {
                 // this launch wrote x0 + dx to the free buffer; the warm start
                 // buffer (x0) takes the third-oldest slot, which held the next

@@ -116,3 +116,47 @@ def test_neumann_direct_selection(gpu):
     f, _ = _film((33, 24, 6), 4, 30.0)                         # 33 = 3 x 11
     with gpu.Film.from_oracle_film(f, precision=gpu.FP32_REFINED) as g:
         assert g.inner_solver == gpu.INNER_PCG
+
+
+def _smooth_film(shape):
+    """One grain, P a wave of one period along x: a potential of the longest mode."""
+    nx, ny, nz = shape
+    f, _ = _film(shape, 3, 30.0)
+    f.omega = np.zeros(f.N, np.int32)
+    f.grain_mat, f.TR = np.ones(1, np.int32), np.asarray(f.TR).reshape(-1, 9)[:1].reshape(-1)
+    f.is_interface = np.zeros(f.N, np.int32)
+    x = np.tile(np.arange(nx), ny * nz)
+    return f, [0.2 * np.sin(2 * np.pi * x / nx + q) for q in range(6)]
+
+
+@pytest.mark.parametrize("shape", [(512, 32, 5), (32, 256, 4)])
+def test_neumann_direct_long_modes(gpu, shape):
+    """The FP32 check of a step sees modes of a whole side as they are: one more
+    solve removes what the first one rounded off, and no further one runs on
+    rounding of the check itself (three passes a step at most)."""
+    f, P = _smooth_film(shape)
+    f.del_t = 2e-3
+    with gpu.Film.from_oracle_film(f, precision=gpu.FP32_REFINED, **KW) as g:
+        assert g.inner_solver == gpu.INNER_DIRECT
+        g.set_state(P)
+        g.run(np.linspace(0.0, 0.3, 16))
+        it, rf = g.iters()
+        g.sync()
+    assert (it <= 2).all() and (rf <= 3).all()
+
+
+@pytest.mark.parametrize("tol", [1e-10, 1e-11, 1e-12])
+@pytest.mark.parametrize("shape", [(64, 96, 5), (27, 48, 12)])
+def test_neumann_direct_tight_target(gpu, shape, tol):
+    """A target below what an update from 1e-4 ||b|| rounds off is met by b - A phi."""
+    f, P = _film(shape, 9, 30.0)
+    with gpu.Film.from_oracle_film(f, precision=gpu.FP32_REFINED, refine_tol=tol, max_refine=20) as g:
+        g.set_state(P)
+        assert g.depol()["status"] == 0
+        Pg, phi = g.get_state()
+    b = -oracle.load().divergence(f, Pg[0], Pg[1], Pg[2])
+    r = b - oracle.load().apply_A(f, phi)
+    pin = f.nx // 2 + f.nx * (f.ny // 2 + f.ny * (f.nz // 2))
+    b[pin], r[pin] = 0.0, 0.0
+    # a full pass forms r to 2^-48 of terms up to (96 / 2 pi)^2 of it: 8e-13 at worst, a tenth of that in the mean square
+    assert np.linalg.norm(r) <= 1.1 * tol * np.linalg.norm(b)
