@@ -1468,6 +1468,10 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
             double len = dsc->nz / M_PI;
             if (dsc->zbc != CMSL_DIRICHLET) len = std::max(len, std::max(dsc->nx, dsc->ny) / (2.0 * M_PI));
             fd.upd_c = fd.uni_eps && dsc->zbc == CMSL_DIRICHLET ? 0.f : (float)(4.0 * std::ldexp(1.0, -24) * std::max(1.0, len));
+            // a target near what the stored potential's 48 bits leave in its
+            // residual (the smoothest mode's phi / h^2 is len^2 of b) takes full
+            // passes only: they see that rounding (512x256x8 Neumann: 2e-12)
+            if (fd.upd_c > 0.f && dsc->refine_tol < std::ldexp(len * len, -47)) fd.upd_ok = 0;
             fd.refine_tolf = (float)std::sqrt(fd.refine_tol2);
         }
         fd.defer_ok = fd.upd_ok && fd.uni_eps && fd.dep_flag && fd.warm <= 2 ? 1 : 0;

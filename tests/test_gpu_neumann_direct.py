@@ -160,3 +160,20 @@ def test_neumann_direct_tight_target(gpu, shape, tol):
     b[pin], r[pin] = 0.0, 0.0
     # a full pass forms r to 2^-48 of terms up to (96 / 2 pi)^2 of it: 8e-13 at worst, a tenth of that in the mean square
     assert np.linalg.norm(r) <= 1.1 * tol * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("tol", [1e-12, 3e-13, 1e-13])
+def test_neumann_direct_target_below_the_potentials_bits(gpu, tol):
+    """Where the stored potential's 48 bits do not resolve the target, the solve
+    says so (status 3) unless b - A phi meets it."""
+    f, _ = _smooth_film((512, 64, 6))
+    P = list(np.random.default_rng(2).uniform(-0.2, 0.2, (6, f.N)))
+    with gpu.Film.from_oracle_film(f, precision=gpu.FP32_REFINED, refine_tol=tol, max_refine=8) as g:
+        g.set_state(P)
+        status = g.depol()["status"]
+        Pg, phi = g.get_state()
+    b = -oracle.load().divergence(f, Pg[0], Pg[1], Pg[2])
+    r = b - oracle.load().apply_A(f, phi)
+    pin = f.nx // 2 + f.nx * (f.ny // 2 + f.ny * (f.nz // 2))
+    b[pin], r[pin] = 0.0, 0.0
+    assert status == 3 or np.linalg.norm(r) <= 1.1 * tol * np.linalg.norm(b)
