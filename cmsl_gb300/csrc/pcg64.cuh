@@ -124,7 +124,7 @@ constexpr long long FX_BAD = 1ll << 43;             // sound: |top word| <= 2^33
 
 __device__ __forceinline__ int fx_exponent(double ref)
 {
-    return max((int)((__double2hiint(ref) >> 20) & 0x7ff) - 1023 - 100, -1000);
+    return max((int)((__double2hiint(ref) >> 20) & 0x7ff) - 1023 - 100, -1074);     // 2^-1074: the least double
 }
 __device__ __forceinline__ void fx_split(double v, int E, int (&p)[FX_PIECES], bool &bad)
 {
@@ -168,7 +168,9 @@ __device__ __forceinline__ double fx_double(long long lo, long long mid, long lo
     const int lz = __clzll((long long)w2);
     const unsigned long long m = lz ? (w2 << lz) | (w1 >> (64 - lz)) : w2;
     const double v = __ull2double_rn(m);            // in [2^63, 2^64]
-    const double s = __hiloint2double(__double2hiint(v) + ((e - lz) << 20), __double2loint(v));
+    const int k = e - lz, be = (__double2hiint(v) >> 20) + k;
+    // the exponent moved by an integer addition where the result is a normal number
+    const double s = be >= 1 && be <= 2046 ? __hiloint2double(__double2hiint(v) + k * (1 << 20), __double2loint(v)) : ldexp(v, k);
     return neg ? -s : s;
 }
 
@@ -273,17 +275,6 @@ __device__ __forceinline__ bool p64_allreduce(const Pcg64 &B, FxRed &R, int nb, 
     return true;
 }
 
-// a / b (b positive and normal) from the hardware's reciprocal estimate and
-// one third-order step, to about an ulp (the scalars need no more): four
-// dependent FP64 operations, where the compiled division takes 750 cycles.
-__device__ __forceinline__ double p64_div(double a, double b)
-{
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(b));
-    const double e = fma(-b, r, 1.0);
-    return a * fma(r, fma(e, e, e), r);
-}
-
 // The scalars of a film's solve, the same in every block (thread 0 steps them).
 struct P64Scal {
     double alpha, beta, rz, rr;
@@ -295,7 +286,7 @@ __device__ __forceinline__ void p64_after_s(P64Scal &s, bool ok, double pq, bool
 {
     const bool good = ok && isfinite(pq) && pq > 0.0;
     s.go = !ok ? -1 : good || force ? 1 : -2;
-    s.alpha = force ? 1e-3 : p64_div(s.rz, pq);
+    s.alpha = force ? 1e-3 : s.rz / pq;
 }
 // After U (thread 0): beta and the stop test (depol_varEPS.cu:508-521, :472-474).
 __device__ __forceinline__ void p64_after_u(P64Scal &s, const FilmDev *f, bool ok, double rzn, double rrn, int iters,
@@ -306,7 +297,7 @@ __device__ __forceinline__ void p64_after_u(P64Scal &s, const FilmDev *f, bool o
     else if (!isfinite(rzn) || rzn < 0.0) s.go = -2;
     else if (f->crit == 0) s.go = iters < max_iter && rzn > f->tol_abs2 && (rz0 <= 0.0 || rzn / rz0 > f->tol_rel2);
     else s.go = iters < max_iter && rrn > f->tol_rel2 * bb;
-    s.beta = force ? 0.5 : p64_div(rzn, s.rz);
+    s.beta = force ? 0.5 : rzn / s.rz;
     s.rz = rzn;
     s.rr = rrn;
 }

@@ -147,3 +147,23 @@ def test_pcg64_wait_timeout_ends_single_calls(gpu, form, monkeypatch):
         with pytest.raises(gpu.CmslError) as e:
             g.loop_gradient(np.full(2, 0.1), np.arange(2, dtype=np.int32), np.zeros(2), 2)
         assert e.value.status == 2 and "barrier timed out" in str(e.value)
+
+
+@pytest.mark.parametrize("form", ["resident", "streaming"])
+@pytest.mark.parametrize("k", [-490, -470, -300, 400, 500])
+def test_pcg64_over_the_exponent_range(gpu, form, k, monkeypatch):
+    """P scaled by 2^k scales the solve exactly: the sums and their quotients
+    hold down to subnormal r.z (2^k = 2^-490: 2^-977 at the start, 2^-1037 at
+    the end, with 37 bits left) and up to 2^1003."""
+    monkeypatch.setenv("CMSL_P64_STREAM", "1" if form == "streaming" else "0")
+    f, P = random_film(64, 32, 8, seed=72, eps_0_nd=3.0)
+    f.crit, f.tol_rel, f.max_iter = oracle.CRIT_RELRES, 1e-9, 4000
+    out = []
+    for s in (1.0, 2.0 ** k):
+        with gpu.Film.from_oracle_film(f) as g:
+            g.set_state([p * s for p in P])
+            res = g.depol()
+            assert res["status"] == 0
+            out.append((res["iters"], g.get_state()[1] / s))
+    assert out[0][0] == out[1][0]
+    assert np.abs(out[0][1] - out[1][1]).max() <= 1e-10 * np.abs(out[0][1]).max()
