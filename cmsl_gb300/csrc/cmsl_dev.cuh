@@ -94,7 +94,7 @@ struct FilmDev {
     int defer_ok;               // the check after a step's one direct solve may run inside the next
                                 // TDGL step (upd_ok, one eps, warm start at most quadratic)
     double n_mat[3];            // voxels per material (sum of the reference's masks)
-    double rowc[11];            // sweep row: factors of the sums, constants (evolve.cu:391-400)
+    double rowc[11];            // sweep row: 1 / cells, voxels a material's sum is divided by, constants (evolve.cu:391-400)
     Coef<double> coef[6];       // index mat*2 + iface
     Coef<float> coef32[6];
     float coef_rot[6][12];      // the FP32 step's combined coefficients for orthonormal rotations (tdgl_cell32)

@@ -1607,7 +1607,7 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
         static const int mat[3] = {1, 0, 2};                 // row order FE, AFE, DE
         for (int q = 0; q < 3; ++q) {
             const double nm = fd.n_mat[mat[q]];
-            fd.rowc[4 + 2 * q] = nm > 0.0 ? 1.0 / nm : 0.0;
+            fd.rowc[4 + 2 * q] = nm;
             fd.rowc[5 + 2 * q] = nm > 0.0 ? nm / N : 0.0;
         }
         fd.rowc[10] = 0.0;

@@ -638,14 +638,17 @@ __global__ void __launch_bounds__(NT) k_tdgl(Dev d, Fields<T> F)
 // sums (evolve.cu:256-357 scaled as in :391-400), and the per-step reset of
 // the solver state.
 // Film fi's sweep row frow from the totals of its seven row sums (thread q < 11
-// the row's value q; FilmDev::rowc: 1 / voxels, fractions); step: steps done.
+// the row's value q; FilmDev::rowc: 1 / cells, voxels, fractions); step: steps done.
 __device__ __forceinline__ void row_write(const Dev &d, int fi, int frow, const double *tot, int step)
 {
     const int q = threadIdx.x;
     if (q >= 11) return;
     const double c = d.films[fi].rowc[q];
-    const int src = q < 5 ? q : q == 6 ? 5 : q == 8 ? 6 : -1;
-    d.rowbuf[((long long)fi * d.rstride + frow) * 11 + q] = q == 10 ? (double)(step + 1) : src >= 0 ? tot[src] * c : c;
+    double v = c;                                   // fractions
+    if (q < 4) v = tot[q] * c;
+    else if (q == 10) v = (double)(step + 1);
+    else if ((q & 1) == 0) v = c > 0.0 ? tot[q / 2 + 2] / c : 0.0;      // material means
+    d.rowbuf[((long long)fi * d.rstride + frow) * 11 + q] = v;
 }
 
 // Film fi's solver state at the start of a step (one thread).

@@ -261,3 +261,24 @@ def test_checkpoint_restart_continues_the_run(gpu, orc, precision, tmp_path):
     tol = 1e-9 if precision == "fp64" else 2e-5
     for x, y in zip(Pb, Pa):
         assert np.abs(x - y).max() <= tol * np.abs(y).max()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_rows_material_means_divide(gpu, orc, precision):
+    """A material's mean in a sweep row is its sum over its voxels, rounded
+    once (evolve.cu:391-400): P_z = 1 in every cell of a film at rest, with
+    voxel counts n of which n (1 / n) is not 1."""
+    f, _ = random_film(1, 328, 3, seed=3, dep_flag=0)
+    y = np.tile(np.arange(328), 3)
+    f.omega = np.where(y < 83, 0, np.where(y < 249, 1, 2)).astype(np.int32)
+    f.grain_mat, f.TR = np.array([1, 0, 2], np.int32), np.tile(np.eye(3).reshape(-1), 3)
+    f.mats = f.mats.copy()
+    f.mats[:, 5:7] = 0.0                                    # no gradient term, no kinetics: P stays
+    f.is_interface = np.zeros(f.N, np.int32)
+    n = np.array([249, 498, 237])
+    assert (n * (1.0 / n) != 1.0).all()
+    with _film(gpu, f, precision=gpu.FP64 if precision == "fp64" else gpu.FP32_REFINED) as g:
+        g.set_state([np.ones(f.N)] * 6)
+        g.run(np.zeros(2), np.arange(2, dtype=np.int32))
+        r = g.rows()
+    assert (r[:, [4, 6, 8]] == 1.0).all() and (r[:, [5, 7, 9]] == n / f.N).all()
