@@ -85,6 +85,7 @@ struct FilmDev {
     int uni_eps;                // all materials share eps_r
     float cheb_delta;           // direct solve preconditioning several eps: (kappa - 1) / (kappa + 1),
                                 // the half-width of M^-1 A's spectrum around 1 (0: exact solve)
+    double cheb_2d;             // 2 / cheb_delta
     int upd_ok;                 // FP32_REFINED: the inner solve leaves r intact (direct solve), so a
                                 // later refinement pass may update r instead of recomputing it
     float upd_c;                // what an update pass rounds off, relative to ||A dx|| (0: one eps and the
@@ -126,8 +127,8 @@ struct SolveDev {               // per film, lives in device memory
     int inner_max;              // inner iteration cap of the current pass
     int upd;                    // the next refinement pass updates r <- r - A dx (FP32) instead of
                                 // forming b - A phi in double-float
+    double cheb_rho;            // Chebyshev recurrence of the preconditioned refinement (rho_k)
     float upd_err;              // what the updates up to the next pass may have rounded off r, over ||b||
-    float cheb_rho;             // Chebyshev recurrence of the preconditioned refinement (rho_k)
     float cheb_w, cheb_m;       // the next direct solve's increment: dx <- w M^-1 r + m dx
     float pin_r, pin_x;         // direct solve of a Neumann film: r and the previous increment at the pinned cell
     int pending;                // the step ended on its direct solve: the potential is phi_cur (the

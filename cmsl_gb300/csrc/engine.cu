@@ -1476,10 +1476,12 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
         }
         fd.defer_ok = fd.upd_ok && fd.uni_eps && fd.dep_flag && fd.warm <= 2 ? 1 : 0;
         fd.cheb_delta = 0.f;
+        fd.cheb_2d = 0.0;
         if (e->spectral && !fd.uni_eps && fd.dep_flag) {
             double kappa = 1.0;
             spec_eps_ref(*dsc, &kappa);
             fd.cheb_delta = (float)((kappa - 1.0) / (kappa + 1.0));
+            fd.cheb_2d = fd.cheb_delta > 0.f ? 2.0 / (double)fd.cheb_delta : 0.0;
             const int cap = spec_precond_refine_cap(kappa, dsc->refine_tol);
             fd.max_refine = std::max(fd.max_refine, cap);
             e->max_refine_cap = std::max(e->max_refine_cap, cap);

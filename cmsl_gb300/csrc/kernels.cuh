@@ -897,6 +897,7 @@ __device__ __forceinline__ void refine_film(const Dev &d, int fi, FilmTail &T)
     const double tol2 = ff->refine_tol2;
     const int dep = ff->dep_flag, upd_ok = ff->upd_ok, defer_ok = ff->defer_ok, max_refine = ff->max_refine;
     const int direct = ff->direct, inner_max = ff->inner_max;
+    const double twodl = ff->cheb_2d;
     const float dl = ff->cheb_delta, uc = ff->upd_c, tol = ff->refine_tolf;
     if (!dep) return;
     film_tail<3>(d, fi, 1, T);
@@ -944,16 +945,16 @@ __device__ __forceinline__ void refine_film(const Dev &d, int fi, FilmTail &T)
         // direct solve preconditioning several eps, M^-1 A's spectrum in
         // [1 - delta, 1 + delta]): solve 0 of a step dx = M^-1 r, then
         // rho_k = 1 / (2 / delta - rho_{k-1}), dx_k = (2 rho_k / delta) M^-1 r
-        // + rho_k rho_{k-1} dx_{k-1} (weights of FP32 increments, in FP32)
+        // + rho_k rho_{k-1} dx_{k-1} (the recurrence in FP64)
         if (dl <= 0.f || refine == 1) {
             S->cheb_rho = dl;
             S->cheb_w = 1.f;
             S->cheb_m = 0.f;
         } else {
-            const float rp = P.cheb_rho, rk = 1.f / (2.f / dl - rp);
+            const double rp = P.cheb_rho, rk = 1.0 / (twodl - rp);
             S->cheb_rho = rk;
-            S->cheb_w = 2.f * rk / dl;
-            S->cheb_m = rk * rp;
+            S->cheb_w = (float)(twodl * rk);
+            S->cheb_m = (float)(rk * rp);
         }
         S->iters = 0;
         S->rz = S->rz0 = rz;
