@@ -638,11 +638,13 @@ __global__ void __launch_bounds__(NT) k_tdgl(Dev d, Fields<T> F)
 // sums (evolve.cu:256-357 scaled as in :391-400), and the per-step reset of
 // the solver state.
 // Film fi's sweep row frow from the totals of its seven row sums (thread q < 11
-// the row's value q; FilmDev::rowc: 1 / cells, voxels, fractions); step: steps done.
+// of the second warp the row's value q, so that its quotients pass while the
+// first one sets the step up; FilmDev::rowc: 1 / cells, voxels, fractions);
+// step: steps done.
 __device__ __forceinline__ void row_write(const Dev &d, int fi, int frow, const double *tot, int step)
 {
-    const int q = threadIdx.x;
-    if (q >= 11) return;
+    const int q = (int)threadIdx.x - 32;
+    if (q < 0 || q >= 11) return;
     const double c = d.films[fi].rowc[q];
     double v = c;                                   // fractions
     if (q < 4) v = tot[q] * c;

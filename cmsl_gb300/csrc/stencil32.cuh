@@ -533,7 +533,6 @@ __device__ __forceinline__ void tdgl_def_film(const Dev &d, int rs, int fi, Film
         if (frow >= 0) row_write(d, fi, frow, T.tot, T.c.step);
         if (threadIdx.x == 0 && dep && T.S.pending) d.solve[fi].rr64 = T.tot[7];
     }
-    __syncthreads();            // T is the next film's
 }
 
 // A pending film's check passed (NaN fails): the update pass's test, with what
