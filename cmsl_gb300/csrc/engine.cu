@@ -1350,6 +1350,28 @@ template <class Cap> std::vector<int> share_blocks(const Engine *e, int total, C
     return nb;
 }
 
+// The FP32 stencil kernels of a handle: FB batches, UNI one permittivity, ROT
+// orthonormal rotations (films of others apply all nine values of a rotation,
+// by the same tilings, stagings and deferred checks).
+template <bool FB> void refine_kernels(Engine *e, bool uni)
+{
+    constexpr int U = r32_ns<true>(), V = r32_ns<false>();
+    e->refine_cp[0] = uni ? (void *)k_refine32<true, U, 4, FB> : (void *)k_refine32<false, V, 4, FB>;
+    e->refine_cp[1] = uni ? (void *)k_refine32<true, U, 8, FB> : (void *)k_refine32<false, V, 8, FB>;
+    e->refine_cp[2] = uni ? (void *)k_refine32<true, U, 16, FB> : (void *)k_refine32<false, V, 16, FB>;
+    e->refine_tma = uni ? (void *)k_refine32t<true, RT_NS, FB> : (void *)k_refine32t<false, RT_NS, FB>;
+}
+template <bool FB, bool ROT> void tdgl_kernels(Engine *e)
+{
+    e->tdgl_cp[0] = (void *)k_tdgl32<T32_NS, 4, false, FB, ROT>;
+    e->tdgl_cp[1] = (void *)k_tdgl32<T32_NS, 8, false, FB, ROT>;
+    e->tdgl_cp[2] = (void *)k_tdgl32<T32_NS, 16, false, FB, ROT>;
+    e->tdgl_def[0] = (void *)k_tdgl32<T32_NS, 4, true, FB, ROT>;
+    e->tdgl_def[1] = (void *)k_tdgl32<T32_NS, 8, true, FB, ROT>;
+    e->tdgl_def[2] = (void *)k_tdgl32<T32_NS, 16, true, FB, ROT>;
+    e->tdgl_tma = (void *)k_tdgl32t<TT_NS, FB, ROT>;
+}
+
 cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
 {
     for (int i = 0; i < n; ++i) TRY(check_desc(descs + i, i, n));
@@ -1599,7 +1621,7 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
         const char *df = getenv("CMSL_DEFER");
         bool any_def = false;
         for (int fi = 0; fi < n; ++fi) any_def |= fds[fi].defer_ok != 0;
-        e->defer = e->spectral && !e->persistent && e->rot && any_def && !(df && atoi(df) == 0);
+        e->defer = e->spectral && !e->persistent && any_def && !(df && atoi(df) == 0);
     }
     TRY(e->alloc((void **)&e->d_code, sizeof(uint32_t) * cells));
     TRY(build_film_codes(e, descs, fds));
@@ -1631,10 +1653,6 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
         const int ty_env = tyv ? atoi(tyv) : 0;
         e->tile_fixed = e->precision != CMSL_FP64 && (ty_env == 4 || ty_env == 8 || ty_env == 16);
         e->stile_ty = e->tile_fixed ? ty_env : TY;
-        if (!e->rot) {                  // general rotations: one tile shape
-            e->tile_fixed = true;
-            e->stile_ty = TY;
-        }
         std::lock_guard<std::mutex> lk(g_tuned_mu);
         const auto hit = g_tuned.find(shape_key(e));
         if (hit != g_tuned.end()) {
@@ -1945,36 +1963,17 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
         // the cp.async ring for all)
         const char *nt = getenv("CMSL_NO_TMA");
         e->tma = !(nt && atoi(nt) != 0);
-        e->tma = e->tma && e->rot;
         for (int fi = 0; fi < n; ++fi) e->tma = e->tma && e->fh[fi].nx % TX == 0 && e->fh[fi].ny % TY == 0;
         // the cp.async ring at every tile height, the tensor copies at TY
         // rows; batches take the kernels that finish each film in its own
         // last block
         const bool fb = n > 1;
-        if (fb) {
-            e->refine_cp[0] = uni ? (void *)k_refine32<true, r32_ns<true>(), 4, true> : (void *)k_refine32<false, r32_ns<false>(), 4, true>;
-            e->refine_cp[1] = uni ? (void *)k_refine32<true, r32_ns<true>(), 8, true> : (void *)k_refine32<false, r32_ns<false>(), 8, true>;
-            e->refine_cp[2] = uni ? (void *)k_refine32<true, r32_ns<true>(), 16, true> : (void *)k_refine32<false, r32_ns<false>(), 16, true>;
-            e->tdgl_cp[0] = (void *)k_tdgl32<T32_NS, 4, false, true>;
-            e->tdgl_cp[1] = (void *)k_tdgl32<T32_NS, 8, false, true>;
-            e->tdgl_cp[2] = (void *)k_tdgl32<T32_NS, 16, false, true>;
-            e->tdgl_def[0] = (void *)k_tdgl32<T32_NS, 4, true, true>;
-            e->tdgl_def[1] = (void *)k_tdgl32<T32_NS, 8, true, true>;
-            e->tdgl_def[2] = (void *)k_tdgl32<T32_NS, 16, true, true>;
-        } else {
-            e->refine_cp[0] = uni ? (void *)k_refine32<true, r32_ns<true>(), 4> : (void *)k_refine32<false, r32_ns<false>(), 4>;
-            e->refine_cp[1] = uni ? (void *)k_refine32<true, r32_ns<true>(), 8> : (void *)k_refine32<false, r32_ns<false>(), 8>;
-            e->refine_cp[2] = uni ? (void *)k_refine32<true, r32_ns<true>(), 16> : (void *)k_refine32<false, r32_ns<false>(), 16>;
-            e->tdgl_cp[0] = (void *)k_tdgl32<T32_NS, 4>;
-            e->tdgl_cp[1] = (void *)k_tdgl32<T32_NS, 8>;
-            e->tdgl_cp[2] = (void *)k_tdgl32<T32_NS, 16>;
-            e->tdgl_def[0] = (void *)k_tdgl32<T32_NS, 4, true>;
-            e->tdgl_def[1] = (void *)k_tdgl32<T32_NS, 8, true>;
-            e->tdgl_def[2] = (void *)k_tdgl32<T32_NS, 16, true>;
-        }
-        if (!e->rot)                    // the rotations applied in full (tile height TY, no deferred checks)
-            for (void *&fn : e->tdgl_cp)
-                fn = fb ? (void *)k_tdgl32<T32_NS, TY, false, true, false> : (void *)k_tdgl32<T32_NS, TY, false, false, false>;
+        if (fb) refine_kernels<true>(e, uni);
+        else refine_kernels<false>(e, uni);
+        if (fb && e->rot) tdgl_kernels<true, true>(e);
+        else if (fb) tdgl_kernels<true, false>(e);
+        else if (e->rot) tdgl_kernels<false, true>(e);
+        else tdgl_kernels<false, false>(e);
         e->refine_cp_smem[0] = uni ? r32_smem<true, 4>() : r32_smem<false, 4>();
         e->refine_cp_smem[1] = uni ? r32_smem<true, 8>() : r32_smem<false, 8>();
         e->refine_cp_smem[2] = uni ? r32_smem<true, 16>() : r32_smem<false, 16>();
@@ -1994,10 +1993,7 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
         }
         if (e->tma) {
             TRY(make_maps(e));
-            if (fb) e->refine_tma = uni ? (void *)k_refine32t<true, RT_NS, true> : (void *)k_refine32t<false, RT_NS, true>;
-            else e->refine_tma = uni ? (void *)k_refine32t<true, RT_NS> : (void *)k_refine32t<false, RT_NS>;
             e->refine_tma_smem = uni ? rt_smem<true>() : rt_smem<false>();
-            e->tdgl_tma = fb ? (void *)k_tdgl32t<TT_NS, true> : (void *)k_tdgl32t<TT_NS>;
             e->tdgl_tma_smem = TT_SMEM;
             CK(cudaFuncSetAttribute(e->refine_tma, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)e->refine_tma_smem));

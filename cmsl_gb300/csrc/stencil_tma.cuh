@@ -144,7 +144,7 @@ constexpr int TT_PHI = 3 * REG2, TT_CODE = 4 * REG2, TT_STAGE = 4 * REG2 + BODY1
 constexpr size_t TT_SMEM = (size_t)TT_NS * TT_STAGE + 128;
 constexpr int TT_OPS = 3 * 5 + 5 + 1;
 
-template <int NS, bool FB = false>
+template <int NS, bool FB = false, bool ROT = true>
 __global__ void __launch_bounds__(NT, 4) k_tdgl32t(Dev d, Fields<float> F)
 {
     static_assert(NS >= 4, "the ring holds planes k-1, k, k+1 and at least one in flight");
@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(NT, 4) k_tdgl32t(Dev d, Fields<float> F)
     const int4 it = d.sitems[blockIdx.x];
     const FilmDev *f = d.films + it.x;
     const int z0 = it.w & 0xffff, z1 = it.w >> 16;
-    load_coef4<true>(f, sC);
+    load_coef4<ROT>(f, sC);
     const int nx = f->nx, ny = f->ny, nz = f->nz, x0 = it.y, y0 = it.z;
     const int cur = d.ctl->cur, rs = d.ctl->run_step;
     const float mEz = (float)(-d.wave[(long long)it.x * d.wstride + rs]);   // dfdPmz_app, kernels_evol.cu:210
@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(NT, 4) k_tdgl32t(Dev d, Fields<float> F)
     const float2 *uh = phi2_sel(d, S->phi_prev2) + off;
     const float2 *vh = phi2_sel(d, S->phi_prev3) + off;
     float2 *nh = phi2_sel(d, phi_free(S)) + off;
-    const float4 *TR4 = (const float4 *)(F.TR + (long long)TR32_ROT * f->g_off);
+    const float4 *TR4 = (const float4 *)(F.TR + (long long)(ROT ? TR32_ROT : TR32_GEN) * f->g_off);
     float2 *Pn = pairs32(F, cur ^ 1) + off;
     const int zlo = max(z0 - 1, 0), zhi = min(z1, nz - 1);
     const FilmMaps *M = d.maps + it.x;
@@ -244,7 +244,7 @@ __global__ void __launch_bounds__(NT, 4) k_tdgl32t(Dev d, Fields<float> F)
             ez = phi_diff32(pu, pd) * inv_2hf;
         }
         float pn[6], pMZl, pSZl;
-        tdgl_cell32<true>(sC[code_mat(c) * 2 + code_iface(c)], TR4, code_gid(c), pc, sum, ex, ey, ez, mEz, pn, pMZl, pSZl);
+        tdgl_cell32<ROT>(sC[code_mat(c) * 2 + code_iface(c)], TR4, code_gid(c), pc, sum, ex, ey, ez, mEz, pn, pMZl, pSZl);
         #pragma unroll
         for (int j = 0; j < 3; ++j) Pn[j * fs + o] = make_float2(pn[2 * j], pn[2 * j + 1]);
         if (row >= 0) row_acc(acc, code_mat(c), pn, pMZl, pSZl);

@@ -70,3 +70,44 @@ def test_general_rotations_in_a_batch(gpu):
             assert rc == 0
             for a, w in zip(b.get_state(i)[0], Pw):
                 assert np.abs(a - w).max() <= 2e-5 * np.abs(w).max()
+
+
+@pytest.mark.parametrize("setting", [("CMSL_TILE_Y", "4"), ("CMSL_TILE_Y", "16"), ("CMSL_STAGING", "11"), ("CMSL_DEFER", "0")])
+@pytest.mark.parametrize("films", [1, 2])
+def test_single_precision_rotations(gpu, setting, films, monkeypatch):
+    """Rotations that passed through FP32 take the general path by every tile
+    height, staging and form of the check that orthonormal ones have."""
+    monkeypatch.setenv(*setting)
+    if setting[0] == "CMSL_STAGING":
+        monkeypatch.setenv("CMSL_DEFER", "0")                # the tensor-copy TDGL step
+    fs = []
+    for seed in range(films):
+        f, P = _case((96, 24, 7), False, 5 + seed)        # a shape that no other test here tunes
+        f = dataclasses.replace(f, TR=np.asarray(f.TR).astype(np.float32).astype(np.float64), mats=f.mats.copy())
+        f.mats[:, 7] = 30.0
+        f.crit, f.tol_rel, f.max_iter = oracle.CRIT_RELRES, 1e-12, 20000
+        fs.append((f, P))
+    Ez = np.linspace(0.0, 0.3, 10)
+    kw = dict(precision=gpu.FP32_REFINED, refine_tol=1e-8, inner_tol=1e-5)
+    if films == 1:
+        with gpu.Film.from_oracle_film(fs[0][0], **kw) as g:
+            cfg = g.tile_config()
+            g.set_state(fs[0][1])
+            g.run(Ez)
+            got = [g.get_state()[0]]
+    else:
+        with gpu.Batch.from_oracle_films([f for f, _ in fs], **kw) as b:
+            cfg = b.tile_config()
+            for i, (_, P) in enumerate(fs):
+                b.set_state(i, P)
+            assert (b.run(np.stack([Ez] * films)) == 0).all()
+            got = [b.get_state(i)[0] for i in range(films)]
+    if setting[0] == "CMSL_TILE_Y":
+        assert cfg["y"] == int(setting[1])
+    if setting[0] == "CMSL_STAGING":
+        assert cfg["tdgl_staging"] == cfg["residual_staging"] == "tensor copies"
+    for (f, P), Pg in zip(fs, got):
+        Pw, _, _, _, _, rc = oracle.load().run(f, P, np.zeros(f.N), Ez)
+        assert rc == 0
+        for a, w in zip(Pg, Pw):
+            assert np.abs(a - w).max() <= 2e-5 * np.abs(w).max()
