@@ -2254,7 +2254,8 @@ cmsl_status get_iters(Engine *e, int film, int n, int32_t *iters, int32_t *refin
 }
 
 // ms[0] TDGL, ms[1] solve set-up / first refinement pass, ms[2] and ms[3] the
-// PCG kernels (persistent solvers: ms[2] per iteration, ms[3] the step end; direct solve: ms[2] the solve, ms[3] the update pass, 0 under
+// PCG kernels (persistent solvers: ms[2] per iteration, ms[3] a launch of the
+// step end; direct solve: ms[2] the solve, ms[3] the update pass, 0 under
 // deferred checks, whose TDGL kernel forms the check and is timed with every
 // depolarised film pending).  The kernels run in force mode, which leaves the
 // solver state as it is, so every repetition times the same kind of pass; the

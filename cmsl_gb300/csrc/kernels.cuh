@@ -1251,7 +1251,7 @@ __global__ void __launch_bounds__(NT) k_update(Dev d, Fields<T> F)
 // ------------------------------------------------------------ step end
 static __global__ void k_step_end(Dev d)
 {
-    step_end(d);
+    if (!d.force) step_end(d);      // kernel timing: the counters stay as they are
 }
 
 // A fixed pseudo-random P of amplitude 0.05 (FP32 pairs, n floats) for the

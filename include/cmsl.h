@@ -191,10 +191,14 @@ cmsl_status cmsl_film_depol_device(cmsl_film *film, const double *Pmx, const dou
 
 /* Average device time (ms, CUDA events on the launch stream) of each kernel
  * of a step, each launched `reps` times back to back on the current state:
- * ms[0] TDGL step, ms[1] solve set-up (FP64 RHS + r0, or FP32_REFINED FP64
- * residual pass), ms[2] PCG p-update + SpMV + p.Ap, ms[3] PCG x/r update +
- * r.z.  The PCG kernels run with the solve forced active, so the call
- * changes the film's work vectors; run it after the steps being measured. */
+ * ms[0] TDGL step, ms[1] solve set-up (FP64 RHS + r0, or FP32_REFINED
+ * residual pass).  Persistent PCGs (FP64, FP32): ms[2] one iteration, ms[3] a
+ * launch of the step end; two-kernel PCG: ms[2] p-update + SpMV + p.Ap, ms[3]
+ * x/r update + r.z; direct solve: ms[2] the solve, ms[3] the update pass (0
+ * where the next TDGL step forms it).  The PCG kernels run with the solve
+ * forced active, so the call changes the film's work vectors and the FP64
+ * potential; run it after the steps being measured.  P and the step counter
+ * stay as they are. */
 cmsl_status cmsl_film_time_kernels(cmsl_film *film, int reps, void *stream, double *ms);
 
 /* The FP32_REFINED inner solve the film uses: CMSL_INNER_DIRECT or

@@ -167,3 +167,21 @@ def test_pcg64_over_the_exponent_range(gpu, form, k, monkeypatch):
             out.append((res["iters"], g.get_state()[1] / s))
     assert out[0][0] == out[1][0]
     assert np.abs(out[0][1] - out[1][1]).max() <= 1e-10 * np.abs(out[0][1]).max()
+
+
+@pytest.mark.parametrize("reps", [4, 40])
+def test_pcg64_timing_leaves_steps_and_p(gpu, reps):
+    """Kernel timing and tuning advance no step: P, the steps done (row column
+    10) and the log of the last run stay, also for more repetitions than the
+    run had steps."""
+    f, P = random_film(48, 20, 8, seed=6, eps_0_nd=3.0)
+    with gpu.Film.from_oracle_film(f) as g:
+        g.set_state(P)
+        g.run(np.full(3, 0.1), np.arange(3, dtype=np.int32))
+        before, log = g.get_state()[0], g.iters()
+        g.time_kernels(reps=reps)
+        g.autotune()
+        assert all(np.array_equal(a, b) for a, b in zip(before, g.get_state()[0]))
+        assert all(np.array_equal(a, b) for a, b in zip(log, g.iters()))
+        g.run(np.full(1, 0.1), np.zeros(1, np.int32))
+        assert g.rows()[0, 10] == 4
