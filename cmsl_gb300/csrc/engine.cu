@@ -1678,21 +1678,6 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
     TRY(e->alloc(&e->d_p[0], e->esz * cells));
     TRY(e->alloc(&e->d_p[1], e->esz * cells));
     if (e->precision != CMSL_FP64) TRY(e->alloc(&e->d_x, e->esz * cells));
-    if (e->pcg64) {
-        Pcg64 &B = e->p64;
-        TRY(e->alloc((void **)&B.z, sizeof(double) * cells));
-        TRY(e->alloc((void **)&B.op, sizeof(uint32_t) * cells));
-        TRY(e->alloc((void **)&B.words, sizeof(unsigned long long) * P64_WORDS * n));
-        TRY(e->alloc((void **)&B.blk_film, sizeof(int) * blk_film.size()));
-        CK(cudaMemcpy((void *)B.blk_film, blk_film.data(), sizeof(int) * blk_film.size(), cudaMemcpyHostToDevice));
-        TRY(e->alloc((void **)&B.err, sizeof(int)));
-        e->cg.err = B.err;
-        // as for the FP32 persistent solver: shorter waits and a block that
-        // never publishes, for the host test of the timeout
-        const char *sl = getenv("CMSL_PCG_SPIN_LIMIT"), *hb = getenv("CMSL_PCG_HOLD_BLOCK");
-        B.spin_limit = sl && atoll(sl) > 0 ? (unsigned long long)atoll(sl) : P64_SPIN_LIMIT;
-        B.hold_block = hb ? atoi(hb) : -1;
-    }
     if (e->persistent) {
         // persistent single-reduction PCG: r (the shared r), u, w, s; x =
         // correction, p in place
@@ -2018,6 +2003,34 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
             const auto hit = g_tuned.find(shape_key(e));
             if (hit != g_tuned.end()) e->stage(hit->second.stg_tdgl, hit->second.stg_refine);
         }
+    }
+    if (e->pcg64) {
+        // its two vectors come last: films that fill the memory without them
+        // (156 bytes a cell) take the two-kernel loop
+        Pcg64 &B = e->p64;
+        cmsl_status r = e->alloc((void **)&B.z, sizeof(double) * cells);
+        if (r == CMSL_OK) r = e->alloc((void **)&B.op, sizeof(uint32_t) * cells);
+        if (r == CMSL_ERR_NOMEM) {
+            cudaGetLastError();
+            if (B.z) e->release(B.z, sizeof(double) * cells);
+            B = Pcg64{};
+            e->pcg64 = false;
+        } else if (r != CMSL_OK) {
+            return r;
+        }
+    }
+    if (e->pcg64) {
+        Pcg64 &B = e->p64;
+        TRY(e->alloc((void **)&B.words, sizeof(unsigned long long) * P64_WORDS * n));
+        TRY(e->alloc((void **)&B.blk_film, sizeof(int) * blk_film.size()));
+        CK(cudaMemcpy((void *)B.blk_film, blk_film.data(), sizeof(int) * blk_film.size(), cudaMemcpyHostToDevice));
+        TRY(e->alloc((void **)&B.err, sizeof(int)));
+        e->cg.err = B.err;
+        // as for the FP32 persistent solver: shorter waits and a block that
+        // never publishes, for the host test of the timeout
+        const char *sl = getenv("CMSL_PCG_SPIN_LIMIT"), *hb = getenv("CMSL_PCG_HOLD_BLOCK");
+        B.spin_limit = sl && atoll(sl) > 0 ? (unsigned long long)atoll(sl) : P64_SPIN_LIMIT;
+        B.hold_block = hb ? atoi(hb) : -1;
     }
     const Dev d = e->dev(0);
     if (e->precision == CMSL_FP64) k_dinv<double><<<(int)e->items.size(), NT>>>(d, (double *)e->d_dinv);

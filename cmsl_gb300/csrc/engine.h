@@ -209,6 +209,13 @@ struct Engine {
         return d;
     }
 
+    // Gives the last allocation back.
+    void release(void *p, size_t n)
+    {
+        cudaFree(p);
+        allocs.pop_back();
+        bytes -= n;
+    }
     cmsl_status alloc(void **p, size_t n)
     {
         cudaError_t e = cudaMalloc(p, n ? n : 16);

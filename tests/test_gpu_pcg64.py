@@ -185,3 +185,27 @@ def test_pcg64_timing_leaves_steps_and_p(gpu, reps):
         assert all(np.array_equal(a, b) for a, b in zip(log, g.iters()))
         g.run(np.full(1, 0.1), np.zeros(1, np.int32))
         assert g.rows()[0, 10] == 4
+
+
+def test_pcg64_film_without_room_for_its_vectors(gpu):
+    """A film that fits the memory but for the persistent PCG's two vectors (12
+    bytes a cell of 168) takes the two-kernel loop and solves as before."""
+    import torch
+    f, P = random_film(256, 256, 128, seed=8, n_grains=8, eps_0_nd=3.0)
+    f.crit, f.tol_rel, f.max_iter = oracle.CRIT_RELRES, 1e-6, 40
+    with gpu.Film.from_oracle_film(f) as g:
+        need = g.device_bytes()
+        g.set_state(P)
+        want, phi = g.depol(), g.get_state()[1]
+    torch.cuda.empty_cache()
+    free = torch.cuda.mem_get_info()[0]
+    hog = torch.empty(free - need + 6 * f.N, dtype=torch.uint8, device="cuda")
+    try:
+        with gpu.Film.from_oracle_film(f) as g:
+            assert g.device_bytes() < need - 11 * f.N
+            g.set_state(P)
+            res, got = g.depol(), g.get_state()[1]
+    finally:
+        del hog
+        torch.cuda.empty_cache()
+    assert res == want and np.abs(got - phi).max() <= 1e-10 * np.abs(phi).max()
