@@ -196,11 +196,28 @@ std::string shape_key(const Engine *e)
 
 constexpr int SPEC_CHIRP_MAX = 2048;        // longest chirp transform: through 4096 values
 // Columns from which AUTO takes the direct solve at sides other than 2^a 3^b.
-// It is the faster one at every size measured (a step 33x32x6 207 -> 67 us,
-// 50x50x10 313 -> 79, 150x110x21 820 -> 96, 317x311x21 1627 -> 350, 500x500x32
-// 8838 -> 878); smaller films keep the PCG, which is what
-// cmsl_film_inner_solver has always answered for them.
+// With one eps it is the faster one at every size measured (a step of 11x13x5
+// 136 -> 52 us, 30x24x6 172 -> 57, 33x32x6 178 -> 59, 50x50x10 309 -> 72,
+// 150x110x21 818 -> 83, 317x311x21 1645 -> 287); with several, thin films gain
+// less or lose (11x13x5 145 -> 233 us, 17x19x8 213 -> 278, 31x31x20 464 -> 297).
+// The line is the size below which the PCG is what cmsl_film_inner_solver has
+// always answered, not one that the times draw.
 constexpr long long SPEC_CHIRP_COLUMNS = 1024;
+// Several eps, such sides, the Dirichlet boundary: the PCG of a step takes
+// about 3.1 iterations a plane, the preconditioned refinement ln(1e3) / ln(its
+// contraction) solves, 5.6 at kappa = 10/3 and 3.3 at 5/3, of some 7 iterations'
+// time each; by the times below the PCG is the faster one up to 1.5 planes a
+// solve (kappa 10/3, 130x130: 4 planes 368 against 164 us, 8 planes 394 / 344, 10
+// planes 404 / 467; 317x311: 525 / 406 at 6, 837 / 885 at 10; kappa 5/3, 130x130:
+// 238 / 164 at 4, 252 / 249 at 6, 265 / 345 at 8).  Below SPEC_THIN_COLUMNS AUTO
+// has answered DIRECT for thin films too, and keeps to it.
+constexpr long long SPEC_THIN_COLUMNS = 128 * 128;
+bool spec_thin(double kappa, int nz)
+{
+    if (!(kappa > 1.0)) return false;
+    const double s = std::sqrt(kappa);
+    return nz <= 1.5 * std::log(1e3) / std::log((s + 1.0) / (s - 1.0));
+}
 
 // n = 2^a 3^b <= 4096 (the FFT radices of spectral.cuh)
 bool spec_radix_ok(int n)
@@ -1420,7 +1437,7 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
     int spec_mmax = 1;
     {
         bool want = false, forced = false, ok = e->precision != CMSL_FP64, anydep = false, ok_auto = true;
-        bool dirichlet = true, fast = true, chirp = true;
+        bool dirichlet = true, fast = true, chirp = true, thin = false;
         for (int i = 0; i < n; ++i) {
             const cmsl_film_desc &d = descs[i];
             forced |= d.inner_solver == CMSL_INNER_DIRECT;
@@ -1437,13 +1454,14 @@ cmsl_status engine_create(Engine *e, const cmsl_film_desc *descs, int n)
             for (int side : {d.nx, d.ny}) chirp &= spec_radix_ok(side) || (side > 1 && side <= SPEC_CHIRP_MAX);
             chirp &= (long long)d.nx * d.ny >= SPEC_CHIRP_COLUMNS || (spec_radix_ok(d.nx) && spec_radix_ok(d.ny));
             dirichlet &= d.zbc == CMSL_DIRICHLET;
+            thin |= d.zbc == CMSL_DIRICHLET && (long long)d.nx * d.ny >= SPEC_THIN_COLUMNS && spec_thin(kappa, d.nz);
             spec_mmax = std::max(spec_mmax, d.zbc == CMSL_DIRICHLET ? d.nz - 2 : d.nz);
         }
         ok &= anydep && spec_zthreads(spec_mmax) > 0;
         if (forced && !(ok && fast && dirichlet))
             return fail(CMSL_ERR_ARG, "inner_solver DIRECT needs FP32_REFINED films whose depolarisation solves have "
                                       "the Dirichlet z boundary and nx, ny of the form 2^a 3^b <= 4096");
-        e->spectral = ok && want && (forced || (ok_auto && chirp));
+        e->spectral = ok && want && (forced || (ok_auto && chirp && (fast || !thin)));
     }
     int cg_per = 0, cg_nsm = 0;
     e->persistent = e->precision != CMSL_FP64 && !e->spectral && all_dirichlet && n <= CG_MAX_FILMS &&

@@ -96,10 +96,12 @@ typedef struct {
  * 2^a 3^b (<= 4096): an in-plane FFT, a tridiagonal solve along z per mode and
  * the inverse FFT.  CMSL_INNER_AUTO also takes it for the Neumann z boundary
  * (mirrored end rows and the pinned cell solved exactly) and for other sides
- * up to 2048 (chirp transforms) where every such film has nx ny >= 1024;
- * CMSL_INNER_DIRECT still asks for the Dirichlet boundary and 2^a 3^b.  With one permittivity for all materials it is exact for
- * the operator up to FP32 rounding.  With several it solves with one
- * reference permittivity (the middle of the range the film's grains use) and
+ * up to 2048 (chirp transforms) where every such film has nx ny >= 1024 and
+ * none of nx ny >= 16384 is both thin and of several permittivities (nz up to 8
+ * at a ratio of 10/3, 5 at 5/3: the PCG is the faster one);
+ * CMSL_INNER_DIRECT still asks for the Dirichlet boundary and 2^a 3^b.
+ * With one permittivity for all materials it is exact for the operator up to
+ * FP32 rounding.  With several it solves with one reference permittivity (the middle of the range the film's grains use) and
  * preconditions the double-float refinement, whose residual applies the true
  * operator; the refinement's increments follow the Chebyshev semi-iteration
  * for the preconditioned spectrum [2 e_min, 2 e_max] / (e_min + e_max), so

@@ -114,3 +114,26 @@ def test_chirp_selection(gpu):
     f, _ = random_film(35, 30, 6, seed=5, mats=mats)
     with gpu.Film.from_oracle_film(f, **kw) as g:
         assert g.inner_solver == gpu.INNER_PCG
+
+
+def test_chirp_selection_thin_films_of_several_eps(gpu):
+    """Thin films of many columns and several permittivities keep the PCG,
+    which takes few iterations there; alone or beside another ragged film."""
+    def solver(shape, eps, **kw):
+        mats = MATS_DEFAULT.copy()
+        mats[:, 7] = eps
+        f, _ = random_film(*shape, seed=4, n_grains=6, fracs=(0.4, 0.4, 0.2), mats=mats, **kw)
+        f.grain_mat[:3] = [0, 1, 2]
+        return f
+    PCG, DIRECT = gpu.INNER_PCG, gpu.INNER_DIRECT
+    deck, near = [50.0, 30.0, 15.0], [50.0, 30.0, 30.0]                    # ratios 10/3 and 5/3
+    for shape, eps, want in [((130, 131, 4), deck, PCG), ((130, 131, 8), deck, PCG), ((130, 131, 9), deck, DIRECT),
+                             ((130, 131, 5), near, PCG), ((130, 131, 6), near, DIRECT), ((130, 131, 4), 30.0, DIRECT),
+                             ((130, 126, 4), deck, DIRECT), ((128, 128, 4), deck, DIRECT)]:
+        with gpu.Film.from_oracle_film(solver(shape, eps), precision=gpu.FP32_REFINED) as g:
+            assert g.inner_solver == want, (shape, eps)
+    with gpu.Film.from_oracle_film(solver((130, 131, 4), deck, zbc=oracle.NEUMANN), precision=gpu.FP32_REFINED) as g:
+        assert g.inner_solver == DIRECT
+    with gpu.Batch.from_oracle_films([solver((130, 131, 4), deck), solver((35, 44, 5), 30.0)],
+                                     precision=gpu.FP32_REFINED) as b:
+        assert b.inner_solver == PCG
