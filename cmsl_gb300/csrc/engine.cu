@@ -953,7 +953,7 @@ cmsl_status launch_refine(Engine *e, cudaStream_t st, const Dev &d, const Fields
     return CMSL_OK;
 }
 
-// One FP32 TDGL step (k_tdgl32 / k_tdgl32p) launched from the host.
+// One FP32 TDGL step (k_tdgl32 / k_tdgl32t) launched from the host.
 cmsl_status launch_tdgl32(Engine *e, cudaStream_t st, const Dev &d, const Fields<float> &F32)
 {
     Dev dd = d;

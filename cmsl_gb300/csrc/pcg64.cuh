@@ -30,9 +30,10 @@
 //     synchronise only their own blocks: one that has converged leaves, the
 //     others go on.
 //   * Films small enough keep every vector in registers (k_pcg64r): 64x64x16
-//     10.6 -> 6.4 us an iteration, 96x80x20 13.3 -> 8.5, 128x128x16 15.4 -> 13.0.
+//     10.6 -> 6.4 us an iteration, 96x80x20 13.3 -> 8.5, 128x128x16 15.4 -> 13.0
+//     (with fixed alpha and beta; their two quotients add 0.3).
 // One iteration, two kernels in a graph loop before and one launch now:
-// 64x64x16 43 -> 6.4 us, 256x256x32 with three permittivities 190 -> 70 us
+// 64x64x16 43 -> 6.7 us, 256x256x32 with three permittivities 190 -> 71 us
 // (about 15.3 FP64 instructions a cell at the measured 19 cycles each and SM
 // are 61 us).
 //

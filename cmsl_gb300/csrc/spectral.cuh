@@ -367,10 +367,11 @@ __device__ __forceinline__ void stockham_mixed(const float2 *a, float2 *b, int n
 }
 
 // Lengths 2^a 3^b that are no power of two: the passes of pl (spec_plan: the
-// fewest radices of 16, 12, 9, 8, 6, 4, 3, 2 whose product is n -- 96 = 16 x 6
-// and 192 = 16 x 12 take two), between ld and st as fft_pow2.  One radix-2 or
+// fewest radices of 16, 12, 9, 8, 6, 4, 3, 2 whose product is n, the largest as
+// small as it can be -- 96 = 12 x 8 and 192 = 16 x 12 take two), between ld and
+// st as fft_pow2.  One radix-2 or
 // -3 pass through shared memory per factor took 6 to 7 passes: the solve of a
-// 192x96x24 film 56 us, now 33.
+// 192x96x24 film 56 us, now 39.
 template <bool SEQ_FAST, class LD, class ST>
 __device__ __forceinline__ void fft_mixed(float2 *a, float2 *b, int nseq, const SpecAxis &pl, int es, int ss,
                                           const float2 *tw, LD ld, ST st)

@@ -667,9 +667,9 @@ static __global__ void __launch_bounds__(NT) k_extrap(Dev d)
 // as large as phi itself, e.g. the first solve after a cold start).  UNI:
 // every material has the same eps, the operator is eps/h^2 times the 7-point
 // Laplacian (one double-float product per cell, no material codes).
-// An update pass (after the direct solve, once ||r|| <= 1e-4 ||b||) instead
-// forms r <- r - A dx in FP32: dx is then small, and the FP32 rounding of
-// A dx stays far below the refinement target.  With several eps, whose steps
+// An update pass (after the direct solve, once ||r|| <= 1e-4 ||b|| and while
+// its FP32 rounding stays within a quarter of the refinement target,
+// refine_film) instead forms r <- r - A dx in FP32.  With several eps, whose steps
 // take five to eight passes, it reads dx and the codes where the full pass
 // reads the potential, P and D^-1 with halos and works in double-float: 53.4
 // -> 24.7 us a pass at 256x256x32, the step 692 -> 499 us.

@@ -41,8 +41,10 @@ typedef enum { CMSL_DIRICHLET = 0, CMSL_NEUMANN = 1 } cmsl_zbc;
  * CMSL_FP32_REFINED: FP32 fields, stencils and PCG vectors; PCG dots summed in
  *   FP32 within a warp and FP64 above it; the potential is kept in
  *   double-float (two FP32 halves, ~48 significand bits) and an outer
- *   residual-refinement loop evaluated in double-float drives
- *   ||b - A phi|| / ||b|| below refine_tol. */
+ *   residual-refinement loop drives ||b - A phi|| / ||b|| below refine_tol.  Its
+ *   residual is evaluated in double-float, or, after a direct solve of a small
+ *   residual, updated in FP32; what updates may have rounded off is counted
+ *   against refine_tol (several permittivities, Neumann boundary). */
 typedef enum { CMSL_FP64 = 0, CMSL_FP32_REFINED = 1 } cmsl_precision;
 
 /* Stop test of the (inner) PCG.  CMSL_CRIT_REF is the reference's
