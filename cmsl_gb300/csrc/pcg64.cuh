@@ -31,9 +31,10 @@
 //     others go on.
 //   * Films small enough keep every vector in registers (k_pcg64r): 64x64x16
 //     10.6 -> 6.4 us an iteration, 96x80x20 13.3 -> 8.5, 128x128x16 15.4 -> 13.0
-//     (with fixed alpha and beta; their two quotients add 0.3).
+//     (with fixed alpha and beta; their two quotients and the check for a second
+//     all-reduce add 0.5).
 // One iteration, two kernels in a graph loop before and one launch now:
-// 64x64x16 43 -> 6.7 us, 256x256x32 with three permittivities 190 -> 71 us
+// 64x64x16 43 -> 6.9 us, 256x256x32 with three permittivities 190 -> 71 us
 // (about 15.3 FP64 instructions a cell at the measured 19 cycles each and SM
 // are 61 us).
 //
@@ -117,11 +118,15 @@ static __global__ void k_op64(Dev d, uint32_t *op)
 // each to the film's word with one 64-bit atomic.  A word counts the blocks
 // from bit 55 on, so a completed count delivers the sum with the same load.
 // A value that is not finite, or 2^17 above the reference in one thread, puts
-// FX_BAD into the top word, far above what sound blocks can sum to.
+// FX_BAD into the top word, far above what sound blocks can sum to; the blocks,
+// which all see it, then sum once more in units of 2^-40 of the reference (r.z
+// jumps by 2^20 and more where permittivities differ by 1e8), and only a value
+// outside those as well (2^77 above, or not finite) makes the total NaN.
 constexpr int FX_PIECES = 6, FX_BITS = 23, FX_WORDS = 3;
 constexpr int FX_COUNT = 55;                        // first bit of the block count
 constexpr long long FX_BIAS = 1ll << 44;            // keeps the top word's payload positive
 constexpr long long FX_BAD = 1ll << 43;             // sound: |top word| <= 2^33 a block, 2^42 in all
+constexpr int FX_COARSE = 60;                       // the second attempt's units over the first's, as a power of two
 
 __device__ __forceinline__ int fx_exponent(double ref)
 {
@@ -191,12 +196,13 @@ struct FxShared {
 };
 
 // Sums v over the film's blocks, ref: reference values.  tot valid in warp 0
-// of every block, the same bits everywhere (NaN where a value was bad).
+// of every block, the same bits everywhere (all NaN where a value was bad).
 // False in warp 0 after a timeout.  Every thread of the block calls it; the
 // caller's __syncthreads after warp 0's scalar step publishes the outcome.
 // FENCE: the blocks' stores before the call are visible to loads after it
 // (about 600 cycles; not needed where only the sums cross blocks).
-template <int NV, bool FENCE>
+// COARSE: 0, or FX_COARSE for a second attempt.
+template <int NV, bool FENCE, int COARSE = 0>
 __device__ __forceinline__ bool p64_allreduce(const Pcg64 &B, FxRed &R, int nb, FxShared &sm, const double (&v)[NV],
                                               const double (&ref)[NV], double (&tot)[NV])
 {
@@ -206,7 +212,7 @@ __device__ __forceinline__ bool p64_allreduce(const Pcg64 &B, FxRed &R, int nb, 
     #pragma unroll
     for (int i = 0; i < NV; ++i) {
         int p[FX_PIECES];
-        fx_split(v[i], fx_exponent(ref[i]), p, bad);
+        fx_split(v[i], fx_exponent(ref[i]) + COARSE, p, bad);
         #pragma unroll
         for (int j = 0; j < FX_PIECES; ++j) {
             const int s = __reduce_add_sync(0xffffffffu, p[j]);
@@ -264,14 +270,16 @@ __device__ __forceinline__ bool p64_allreduce(const Pcg64 &B, FxRed &R, int nb, 
         }
     }
     if (FENCE) __threadfence();
-    if (R.par) R.prev[1] = w;
-    else R.prev[0] = w;
+    if (own) {                                  // the words of values this call did not sum stay as they were
+        if (R.par) R.prev[1] = w;
+        else R.prev[0] = w;
+    }
     const long long pv = (long long)(diff & ((1ull << FX_COUNT) - 1ull)) - (wi == 2 ? nb * FX_BIAS : 0ll);
     #pragma unroll
     for (int i = 0; i < NV; ++i) {
         const long long lo = __shfl_sync(0xffffffffu, pv, i * FX_WORDS), mid = __shfl_sync(0xffffffffu, pv, i * FX_WORDS + 1);
         const long long hi = __shfl_sync(0xffffffffu, pv, i * FX_WORDS + 2);
-        tot[i] = hi >= FX_BAD / 2 ? __longlong_as_double(0x7ff8000000000000ll) : fx_double(lo, mid, hi, fx_exponent(ref[i]));
+        tot[i] = hi >= FX_BAD / 2 ? __longlong_as_double(0x7ff8000000000000ll) : fx_double(lo, mid, hi, fx_exponent(ref[i]) + COARSE);
     }
     return true;
 }
@@ -279,23 +287,63 @@ __device__ __forceinline__ bool p64_allreduce(const Pcg64 &B, FxRed &R, int nb, 
 // The scalars of a film's solve, the same in every block (thread 0 steps them).
 struct P64Scal {
     double alpha, beta, rz, rr;
-    int go;                     // 1 go on, 0 done, -1 timeout, -2 breakdown
+    int go;                     // 1 go on, 2 sum again in coarse units, 0 done, -1 timeout, -2 breakdown
+    int ok;                     // p64_again: the second attempt's outcome
+    double tot[2];              // and its totals
 };
 
-// After S (thread 0): alpha, or the breakdown of depol_varEPS.cu:486-490.
-__device__ __forceinline__ void p64_after_s(P64Scal &s, bool ok, double pq, bool force)
+// The second attempt of an all-reduce after which the solve would end as a
+// breakdown, out of line: it costs 64x64x16 0.15 us an iteration where a loop
+// around the first attempt cost 0.34.  The outcome goes to sc (valid in thread
+// 0); returns the words' last totals.
+template <int NV>
+__device__ __noinline__ ulonglong2 p64_again(FxRed R, int nb, int *err, unsigned long long spin_limit, int hold_block,
+                                             FxShared *sm, P64Scal *sc, double v0, double v1, double ref0, double ref1)
+{
+    Pcg64 B{};
+    B.err = err;
+    B.spin_limit = spin_limit;
+    B.hold_block = hold_block;
+    double v[NV], ref[NV], tot[NV];
+    v[0] = v0;
+    ref[0] = ref0;
+    if (NV == 2) { v[NV - 1] = v1; ref[NV - 1] = ref1; }
+    const bool ok = p64_allreduce<NV, true, FX_COARSE>(B, R, nb, *sm, v, ref, tot);
+    if (threadIdx.x == 0) {
+        sc->ok = ok;
+        sc->tot[0] = tot[0];
+        sc->tot[1] = tot[NV - 1];
+    }
+    return make_ulonglong2(R.prev[0], R.prev[1]);
+}
+template <int NV>
+__device__ __forceinline__ void p64_second(const Pcg64 &B, FxRed &R, int nb, FxShared &sm, P64Scal &sc, double v0, double v1,
+                                           double ref0, double ref1)
+{
+    const ulonglong2 p = p64_again<NV>(R, nb, B.err, B.spin_limit, B.hold_block, &sm, &sc, v0, v1, ref0, ref1);
+    R.prev[0] = p.x;
+    R.prev[1] = p.y;
+    R.par ^= 1;
+}
+
+// After S (thread 0): alpha, or the breakdown of depol_varEPS.cu:486-490 (bad:
+// 2 after a first attempt, -2 after a second).
+__device__ __forceinline__ void p64_after_s(P64Scal &s, bool ok, double pq, bool force, int bad)
 {
     const bool good = ok && isfinite(pq) && pq > 0.0;
-    s.go = !ok ? -1 : good || force ? 1 : -2;
+    s.go = !ok ? -1 : good || force ? 1 : bad;
     s.alpha = force ? 1e-3 : s.rz / pq;
 }
 // After U (thread 0): beta and the stop test (depol_varEPS.cu:508-521, :472-474).
 __device__ __forceinline__ void p64_after_u(P64Scal &s, const FilmDev *f, bool ok, double rzn, double rrn, int iters,
-                                            int max_iter, double rz0, double bb, bool force)
+                                            int max_iter, double rz0, double bb, bool force, int bad)
 {
     if (!ok) s.go = -1;
     else if (force) s.go = iters < max_iter;
-    else if (!isfinite(rzn) || rzn < 0.0) s.go = -2;
+    else if (!isfinite(rzn) || rzn < 0.0) {
+        s.go = bad;
+        if (bad == 2) return;           // r.z and r.r of the last iteration stay
+    }
     else if (f->crit == 0) s.go = iters < max_iter && rzn > f->tol_abs2 && (rz0 <= 0.0 || rzn / rz0 > f->tol_rel2);
     else s.go = iters < max_iter && rrn > f->tol_rel2 * bb;
     s.beta = force ? 0.5 : rzn / s.rz;
@@ -537,18 +585,33 @@ static __global__ void __launch_bounds__(P64_NT, P64_BPS) k_pcg64(Dev d, Fields<
             else if (R == 2) p64_spmv<2>(G, A, Bv, pn, q, op, first, beta, w0, nw, T, acc[0]);
             else p64_spmv<1>(G, A, Bv, pn, q, op, first, beta, w0, nw, T, acc[0]);
             bool ok = p64_allreduce<1, true>(B, red, nb, sm, acc, ref1, pq);
-            if (threadIdx.x == 0) p64_after_s(sc, ok, pq[0], d.force != 0);
+            if (threadIdx.x == 0) p64_after_s(sc, ok, pq[0], d.force != 0, 2);
             __syncthreads();
-            if (sc.go <= 0) break;
+            if (sc.go != 1) {
+                if (sc.go == 2) {
+                    p64_second<1>(B, red, nb, sm, sc, acc[0], 0.0, sc.rz, 0.0);
+                    if (threadIdx.x == 0) p64_after_s(sc, sc.ok != 0, sc.tot[0], d.force != 0, -2);
+                    __syncthreads();
+                }
+                if (sc.go <= 0) break;
+            }
             double a2[2] = {0.0, 0.0}, tot[2];
             const double ref2[2] = {sc.rz, sc.rr};
             p64_update(n, (long long)lb * P64_NT + threadIdx.x, (long long)nb * P64_NT, x, pn, r, q, dinv, z, sc.alpha,
                        want_rr, a2[0], a2[1]);
             ok = p64_allreduce<2, true>(B, red, nb, sm, a2, ref2, tot);
             ++iters;
-            if (threadIdx.x == 0) p64_after_u(sc, f, ok, tot[0], tot[1], iters, max_iter, rz0, bb, d.force != 0);
+            if (threadIdx.x == 0) p64_after_u(sc, f, ok, tot[0], tot[1], iters, max_iter, rz0, bb, d.force != 0, 2);
             __syncthreads();
-            if (sc.go <= 0) break;
+            if (sc.go != 1) {
+                if (sc.go == 2) {
+                    p64_second<2>(B, red, nb, sm, sc, a2[0], a2[1], sc.rz, sc.rr);
+                    if (threadIdx.x == 0)
+                        p64_after_u(sc, f, sc.ok != 0, sc.tot[0], sc.tot[1], iters, max_iter, rz0, bb, d.force != 0, -2);
+                    __syncthreads();
+                }
+                if (sc.go <= 0) break;
+            }
         }
         if (lb == 0 && threadIdx.x == 0 && !d.force) p64_done(S, sc, iters);
     }
@@ -643,9 +706,16 @@ __device__ __forceinline__ void p64_resident(const Dev &d, const Fields<double> 
             }
         }
         bool ok = p64_allreduce<1, false>(B, red, nb, sm, acc, ref1, pq);
-        if (threadIdx.x == 0) p64_after_s(sc, ok, pq[0], d.force != 0);
+        if (threadIdx.x == 0) p64_after_s(sc, ok, pq[0], d.force != 0, 2);
         __syncthreads();
-        if (sc.go <= 0) break;
+        if (sc.go != 1) {
+            if (sc.go == 2) {
+                p64_second<1>(B, red, nb, sm, sc, acc[0], 0.0, sc.rz, 0.0);
+                if (threadIdx.x == 0) p64_after_s(sc, sc.ok != 0, sc.tot[0], d.force != 0, -2);
+                __syncthreads();
+            }
+            if (sc.go <= 0) break;
+        }
         double a2[2] = {0.0, 0.0}, tot[2];
         const double ref2[2] = {sc.rz, sc.rr}, alpha = sc.alpha;
         #pragma unroll
@@ -663,9 +733,17 @@ __device__ __forceinline__ void p64_resident(const Dev &d, const Fields<double> 
             }
         ok = p64_allreduce<2, true>(B, red, nb, sm, a2, ref2, tot);
         ++iters;
-        if (threadIdx.x == 0) p64_after_u(sc, f, ok, tot[0], tot[1], iters, max_iter, rz0, bb, d.force != 0);
+        if (threadIdx.x == 0) p64_after_u(sc, f, ok, tot[0], tot[1], iters, max_iter, rz0, bb, d.force != 0, 2);
         __syncthreads();
-        if (sc.go <= 0) break;
+        if (sc.go != 1) {
+            if (sc.go == 2) {
+                p64_second<2>(B, red, nb, sm, sc, a2[0], a2[1], sc.rz, sc.rr);
+                if (threadIdx.x == 0)
+                    p64_after_u(sc, f, sc.ok != 0, sc.tot[0], sc.tot[1], iters, max_iter, rz0, bb, d.force != 0, -2);
+                __syncthreads();
+            }
+            if (sc.go <= 0) break;
+        }
         const double beta = sc.beta;
         double ls[ZC], ln[ZC], lx[ZC], lb2[R], lt[R];
         #pragma unroll

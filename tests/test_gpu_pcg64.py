@@ -209,3 +209,33 @@ def test_pcg64_film_without_room_for_its_vectors(gpu):
         del hog
         torch.cuda.empty_cache()
     assert res == want and np.abs(got - phi).max() <= 1e-10 * np.abs(phi).max()
+
+
+@pytest.mark.parametrize("form", ["resident", "streaming"])
+@pytest.mark.parametrize("seed", [9, 27, 32, 35, 38])
+def test_pcg64_sums_far_above_the_last_one(gpu, form, seed, monkeypatch):
+    """Permittivities 1e8 apart: r.z grows by 2^20 and more within an iteration,
+    beyond the units its fixed-point sum starts with."""
+    monkeypatch.setenv("CMSL_P64_STREAM", "1" if form == "streaming" else "0")
+    rng = np.random.default_rng(seed)
+    mats = MATS_DEFAULT.copy()
+    mats[:, 7] = [1e8, 30.0, 1.0]
+    f, _ = random_film(1, 1, 20, seed=1, eps_0_nd=3.0, mats=mats)
+    mat = rng.integers(0, 3, 20)
+    f.omega, f.grain_mat = np.arange(20, dtype=np.int32), mat.astype(np.int32)
+    f.TR = np.tile(np.eye(3).reshape(-1), 20)
+    f.is_interface = np.zeros(20, np.int32)
+    P = list(rng.uniform(-0.2, 0.2, (3, 20))) + [np.zeros(20)] * 3
+    f.crit, f.tol_rel, f.max_iter = oracle.CRIT_RELRES, 1e-9, 4000
+    want, _, _, info = oracle.load().depol_field(f, P[:3], np.zeros(20))
+    assert info["status"] == 0 and info["iters"] < 200
+    with gpu.Film.from_oracle_film(f) as g:
+        g.set_state(P)
+        res = g.depol()
+        phi = g.get_state()[1]
+    # the PCG of a system of condition 1e8 leaves its iterates to rounding: only the solution is compared
+    assert res["status"] == 0 and res["iters"] < 400
+    r = -oracle.load().divergence(f, *P[:3])
+    r[[0, -1]] = 0.0
+    b = np.linalg.norm(r)
+    assert np.linalg.norm(r - oracle.load().apply_A(f, phi)) <= 1e-7 * b
